@@ -42,7 +42,7 @@ def build_ref(source_root: str | None = None) -> str | None:
     present; elsewhere (a GPU box gets the prebuilt library) return the
     library path if it exists, else None."""
     root = source_root or os.environ.get("ARTISYNTH_REFERENCE")
-    if root and os.path.isdir(root):
+    if root and os.path.isfile(os.path.join(root, "src/maspack/solvers/lib/cudssBridgeKernels.cu")):
         subprocess.run(["make", "-s", "-C", _HERE, "ref", "REF=" + root], check=True)
     return REF_LIB_PATH if os.path.exists(REF_LIB_PATH) else None
 
