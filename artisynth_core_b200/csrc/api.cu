@@ -772,6 +772,14 @@ int build_pack(Engine& eng) {
     eng.pcg_row_lanes = bpr <= 40 ? 4 : 16;
   }
 
+  // ---- one team of CTAs per model (pcg_team.cu) wherever every model's rows
+  // fit the shared memory of the CTAs; the split above serves the rest and
+  // the layouts asked for explicitly
+  TeamHost team;
+  eng.team = eng.opt_split == 0 && eng.opt_resident != 1 &&
+             plan_team(eng, gmax, prow, eng.factored ? s1_col : col, eng.factored ? s1_diag : blk_diag,
+                       eng.factored && !dil_nodes.empty(), team);
+
   // ---- device upload
   CK(upload(eng, &d.x, x));
   CK(dalloc(eng, &d.v, 3 * (size_t)N));
@@ -963,6 +971,53 @@ int build_pack(Engine& eng) {
       CK(upload(eng, &d.model_scal2, ms));
     }
   }
+  if (eng.team) {
+    eng.team_grid = team.grid;
+    eng.team_smem = team.smem;
+    eng.team_lanes = team.lanes;
+    eng.team_sets = team.sets;
+    d.team_slots = (int)team.slots.size();
+    CK(upload(eng, &d.team_slot, team.slots));
+    CK(upload(eng, &d.team_rows, team.rows));
+    CK(upload(eng, &d.team_pub, team.pub));
+    CK(upload(eng, &d.team_src, team.src));
+    CK(upload(eng, &d.team_dloc, team.dloc));
+    CK(upload(eng, &d.team_ro, team.ro));
+    CK(upload(eng, &d.team_halo, team.halo));
+    CK(upload(eng, &d.team_cl, team.cl));
+    CK(dalloc(eng, &d.team_ticket, 1));
+    CK(cudaMemset(d.team_ticket, 0, sizeof(unsigned long long)));
+    // cleared packets (tag 0) belong to no exchange: the first tag is 1
+    CK(dalloc(eng, &d.team_base, (size_t)M));
+    CK(cudaMemset(d.team_base, 0, sizeof(unsigned) * (size_t)M));
+    CK(dalloc(eng, &d.team_row_pk, 8 * (size_t)R));
+    CK(cudaMemset(d.team_row_pk, 0, sizeof(double) * 8 * (size_t)R));
+    CK(dalloc(eng, &d.team_part_pk, 8 * team.slots.size()));
+    CK(cudaMemset(d.team_part_pk, 0, sizeof(double) * 8 * team.slots.size()));
+    if (eng.factored && !dil_nodes.empty()) {
+      CK(dalloc(eng, &d.team_t_pk, 4 * (size_t)R));
+      CK(cudaMemset(d.team_t_pk, 0, sizeof(double) * 4 * (size_t)R));
+      // per direct block (row node i, column node j): d_i's entry of j and
+      // d_j's entry of i
+      auto slot_in = [&](int n, int node) -> int {
+        if (eng.hosts[node_model[n]].incomp != B200FEM_INCOMP_NODAL) return -1;
+        auto b = nbr_idx.begin() + nbr_ptr[n], e = nbr_idx.begin() + nbr_ptr[n + 1];
+        auto it = std::lower_bound(b, e, node);
+        return it != e && *it == node ? (int)(it - nbr_idx.begin()) : -1;
+      };
+      std::vector<int> g1(team.blk.size()), g2(team.blk.size());
+      for (size_t i = 0, q = 0; i < team.rows.size(); i++) {
+        const int r = team.rows[i], ni = act_node[r];
+        for (int p = s1_rowptr[r]; p < s1_rowptr[r + 1]; p++, q++) {
+          const int nj = act_node[s1_col[p]];
+          g1[q] = slot_in(ni, nj);
+          g2[q] = slot_in(nj, ni);
+        }
+      }
+      CK(upload(eng, &d.team_g1, g1));
+      CK(upload(eng, &d.team_g2, g2));
+    }
+  }
   CK(dalloc(eng, &d.barrier, 2));
   CK(cudaMemset(d.barrier, 0, 2 * sizeof(unsigned)));
   CK(dalloc(eng, &d.flags, 4));
@@ -980,6 +1035,7 @@ int build_pack(Engine& eng) {
   }
   CK(prepare_kernels(eng));
   CK(prepare_pcg(eng));
+  if (eng.team) CK(prepare_team(eng));
   eng.built = true;
   return B200FEM_OK;
 }
@@ -1725,6 +1781,7 @@ static int read_step_status(Engine& eng, b200fem_stats* stats, int max_iter, boo
   std::memcpy(&st.min_detJ, &bits, sizeof(double));
   eng.last_stats = st;
   if (stats) *stats = st;
+  if (flags[0] != 0) CK(team_recover(eng));
   if (flags[0] == B200FEM_ERR_TIMEOUT) return fail(&eng, B200FEM_ERR_TIMEOUT, "PCG grid barrier timed out");
   if (flags[0] != 0) return fail(&eng, flags[0], "singular diagonal block in the solve matrix");
   if (flags[2] != 0 || !all_conv) {

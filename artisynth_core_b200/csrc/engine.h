@@ -110,6 +110,15 @@ struct ModelHost {
 
 // Device arrays for the whole pack.  Precision-dependent value arrays are
 // allocated in both FP64 and (for the mixed form) FP32.
+
+// One CTA's share of a model in the team PCG (pcg_team.cu): offsets into the
+// slot-major arrays of DevPack.
+struct TeamSlot {
+  int model, rank, k, s0;   // k CTAs in the team, whose first slot is s0
+  int nloc, nh, nb;         // owned rows, rows of other slots it reads, blocks
+  int r0, ro0, h0, b0;      // its first row, row offset, halo row, block
+};
+
 struct DevPack {
   int n_models = 0;
   int n_nodes = 0, n_elems = 0, n_rows = 0;
@@ -265,6 +274,23 @@ struct DevPack {
   double* K_red = nullptr;
   double* crs_red = nullptr;
   double* row_off = nullptr;   // per row: the plane's offset
+  // team PCG (pcg_team.cu), slot-major arrays
+  TeamSlot* team_slot = nullptr;
+  int team_slots = 0;
+  unsigned long long* team_ticket = nullptr;
+  int* team_rows = nullptr;    // owned rows
+  unsigned char* team_pub = nullptr;  // per owned row: another slot reads it
+  int* team_src = nullptr;     // per owned row: its first block in S
+  unsigned short* team_dloc = nullptr;  // per owned row: its diagonal block within the row
+  int* team_ro = nullptr;      // block offsets within the slot (nloc + 1 each)
+  int* team_halo = nullptr;
+  unsigned short* team_cl = nullptr;  // per block: local column
+  int* team_g1 = nullptr;      // factored NODAL: divBlk slots per block
+  int* team_g2 = nullptr;
+  unsigned* team_base = nullptr;   // per model: packet tags used so far
+  double* team_row_pk = nullptr;   // [2][n_rows] two packets of 16 bytes each
+  double* team_part_pk = nullptr;  // [2][slots] two packets each
+  double* team_t_pk = nullptr;     // [2][n_rows]
   // refinement sweeps: FP64 residual, correction, its PCG results
   double* rref = nullptr;
   double* dsol = nullptr;
@@ -352,6 +378,9 @@ struct Engine {
   int pcg_strided = 0;  // pieces dealt to CTAs across models (large packs)
   bool pcg_cluster = false;  // one thread-block cluster per model (pcg_cluster.cu)
   int cl_clusters = 0;       // clusters resident at once
+  bool team = false;         // one team of CTAs per model (pcg_team.cu)
+  int team_grid = 0, team_lanes = 8, team_sets = 1;
+  size_t team_smem = 0;
   int pcg_every_cta_rows = 0;  // every CTA of the PCG split holds at least one piece
   // plane constraints (b200fem_set_plane_constraints): per constrained node
   // its unit normal and offset; enforced by the ConstrainedBackwardEuler step
@@ -445,6 +474,22 @@ cudaError_t launch_attach_reduce(Engine& eng);
 int pcg_cluster_capacity(bool fp32);
 cudaError_t launch_pcg_cluster(Engine& eng, int max_iter, bool update_state, const double* rhs, double* xsol,
                                double tol_override, double* model_out);
+
+// pcg_team.cu: the pack's rows dealt to teams of CTAs (slot-major arrays)
+struct TeamHost {
+  std::vector<TeamSlot> slots;
+  std::vector<int> rows, ro, halo, src, blk;  // blk: per block its index in the pattern
+  std::vector<unsigned short> cl, dloc;
+  std::vector<unsigned char> pub;
+  int nloc = 0, grid = 0, lanes = 8, sets = 1;
+  size_t smem = 0;
+};
+bool plan_team(Engine& eng, int grid_max, const std::vector<int>& rowptr, const std::vector<int>& col,
+               const std::vector<int>& diag, bool dil, TeamHost& out);
+cudaError_t prepare_team(Engine& eng);
+cudaError_t team_recover(Engine& eng);
+cudaError_t launch_pcg_team(Engine& eng, int max_iter, bool update_state, const double* rhs, double* xsol,
+                            double tol_override, double* model_out);
 
 // kernels.cu
 cudaError_t launch_assemble(Engine& eng, double cK, double cM, bool want_K);
