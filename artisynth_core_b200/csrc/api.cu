@@ -974,17 +974,17 @@ int build_pack(Engine& eng) {
   if (eng.team) {
     eng.team_grid = team.grid;
     eng.team_smem = team.smem;
-    eng.team_lanes = team.lanes;
     eng.team_sets = team.sets;
     d.team_slots = (int)team.slots.size();
     CK(upload(eng, &d.team_slot, team.slots));
     CK(upload(eng, &d.team_rows, team.rows));
     CK(upload(eng, &d.team_pub, team.pub));
-    CK(upload(eng, &d.team_src, team.src));
-    CK(upload(eng, &d.team_dloc, team.dloc));
-    CK(upload(eng, &d.team_ro, team.ro));
+    CK(upload(eng, &d.team_diag, team.diag));
     CK(upload(eng, &d.team_halo, team.halo));
+    CK(upload(eng, &d.team_group, team.group));
+    CK(upload(eng, &d.team_blk, team.blk));
     CK(upload(eng, &d.team_cl, team.cl));
+    CK(dalloc(eng, &d.team_stream, (size_t)std::max(team.stream, 1) * team.step_bytes));
     CK(dalloc(eng, &d.team_ticket, 1));
     CK(cudaMemset(d.team_ticket, 0, sizeof(unsigned long long)));
     // cleared packets (tag 0) belong to no exchange: the first tag is 1
@@ -1005,15 +1005,20 @@ int build_pack(Engine& eng) {
         auto it = std::lower_bound(b, e, node);
         return it != e && *it == node ? (int)(it - nbr_idx.begin()) : -1;
       };
-      std::vector<int> g1(team.blk.size()), g2(team.blk.size());
-      for (size_t i = 0, q = 0; i < team.rows.size(); i++) {
-        const int r = team.rows[i], ni = act_node[r];
-        for (int p = s1_rowptr[r]; p < s1_rowptr[r + 1]; p++, q++) {
-          const int nj = act_node[s1_col[p]];
-          g1[q] = slot_in(ni, nj);
-          g2[q] = slot_in(nj, ni);
+      std::vector<int> d_row(s1_col.size()), d_col(s1_col.size());
+      team_parallel((R + 1023) / 1024, [&](int c) {
+        for (int r = 1024 * c; r < std::min(R, 1024 * (c + 1)); r++)
+          for (int p = s1_rowptr[r]; p < s1_rowptr[r + 1]; p++) {
+            d_row[p] = slot_in(act_node[r], act_node[s1_col[p]]);
+            d_col[p] = slot_in(act_node[s1_col[p]], act_node[r]);
+          }
+      });
+      std::vector<int> g1(team.blk.size(), -1), g2(team.blk.size(), -1);
+      for (size_t q = 0; q < team.blk.size(); q++)
+        if (team.blk[q] >= 0) {
+          g1[q] = d_row[team.blk[q]];
+          g2[q] = d_col[team.blk[q]];
         }
-      }
       CK(upload(eng, &d.team_g1, g1));
       CK(upload(eng, &d.team_g2, g2));
     }

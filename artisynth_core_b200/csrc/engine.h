@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -114,9 +115,12 @@ struct ModelHost {
 // One CTA's share of a model in the team PCG (pcg_team.cu): offsets into the
 // slot-major arrays of DevPack.
 struct TeamSlot {
-  int model, rank, k, s0;   // k CTAs in the team, whose first slot is s0
-  int nloc, nh, nb;         // owned rows, rows of other slots it reads, blocks
-  int r0, ro0, h0, b0;      // its first row, row offset, halo row, block
+  int model, rank, k, s0;   // member `rank` of a team of k CTAs, whose first slot is s0
+  int nloc, nh;             // owned rows, rows of other slots it reads
+  int groups, steps;        // row groups of the product and their warp steps
+  int steps_smem;           // steps of S kept in shared memory (the rest streams)
+  int r0, h0, g0, w0;       // its first row, halo row, group entry, step
+  int stream0;              // its first step in the stream
 };
 
 struct DevPack {
@@ -280,12 +284,13 @@ struct DevPack {
   unsigned long long* team_ticket = nullptr;
   int* team_rows = nullptr;    // owned rows
   unsigned char* team_pub = nullptr;  // per owned row: another slot reads it
-  int* team_src = nullptr;     // per owned row: its first block in S
-  unsigned short* team_dloc = nullptr;  // per owned row: its diagonal block within the row
-  int* team_ro = nullptr;      // block offsets within the slot (nloc + 1 each)
+  int* team_diag = nullptr;    // per owned row: its diagonal block in S
   int* team_halo = nullptr;
-  unsigned short* team_cl = nullptr;  // per block: local column
-  int* team_g1 = nullptr;      // factored NODAL: divBlk slots per block
+  int4* team_group = nullptr;  // row groups (pcg_team.cu: RowGroup)
+  int* team_blk = nullptr;     // per step and lane: block of S (-1 none)
+  unsigned short* team_cl = nullptr;  // per step and lane: local column
+  unsigned char* team_stream = nullptr;  // steps beyond the slots' shared memory
+  int* team_g1 = nullptr;      // factored NODAL: divBlk slots per step and lane
   int* team_g2 = nullptr;
   unsigned* team_base = nullptr;   // per model: packet tags used so far
   double* team_row_pk = nullptr;   // [2][n_rows] two packets of 16 bytes each
@@ -379,7 +384,7 @@ struct Engine {
   bool pcg_cluster = false;  // one thread-block cluster per model (pcg_cluster.cu)
   int cl_clusters = 0;       // clusters resident at once
   bool team = false;         // one team of CTAs per model (pcg_team.cu)
-  int team_grid = 0, team_lanes = 8, team_sets = 1;
+  int team_grid = 0, team_sets = 1;
   size_t team_smem = 0;
   int pcg_every_cta_rows = 0;  // every CTA of the PCG split holds at least one piece
   // plane constraints (b200fem_set_plane_constraints): per constrained node
@@ -478,14 +483,17 @@ cudaError_t launch_pcg_cluster(Engine& eng, int max_iter, bool update_state, con
 // pcg_team.cu: the pack's rows dealt to teams of CTAs (slot-major arrays)
 struct TeamHost {
   std::vector<TeamSlot> slots;
-  std::vector<int> rows, ro, halo, src, blk;  // blk: per block its index in the pattern
-  std::vector<unsigned short> cl, dloc;
+  std::vector<int> rows, halo, diag, blk;
+  std::vector<int4> group;
+  std::vector<unsigned short> cl;
   std::vector<unsigned char> pub;
-  int nloc = 0, grid = 0, lanes = 8, sets = 1;
+  int grid = 0, sets = 1, stream = 0, step_bytes = 0;
   size_t smem = 0;
 };
 bool plan_team(Engine& eng, int grid_max, const std::vector<int>& rowptr, const std::vector<int>& col,
                const std::vector<int>& diag, bool dil, TeamHost& out);
+// f(i) for i in [0, n) on the host's threads
+void team_parallel(int n, const std::function<void(int)>& f);
 cudaError_t prepare_team(Engine& eng);
 cudaError_t team_recover(Engine& eng);
 cudaError_t launch_pcg_team(Engine& eng, int max_iter, bool update_state, const double* rhs, double* xsol,

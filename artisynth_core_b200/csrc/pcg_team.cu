@@ -6,8 +6,9 @@
 // (5 us per iteration on the 40x10x10 hex beam whose arithmetic takes well
 // under one).  Here a model's rows are dealt to a team of k CTAs, a compact
 // set of rows each (recursive bisection of the node positions), and
-//   * the CTA's blocks of S stay in shared memory for the whole solve and the
-//     PCG vectors of a row in the registers of the thread that owns it;
+//   * the CTA's blocks of S stay in registers and shared memory for the whole
+//     solve (what exceeds them is streamed from a copy in the order the lanes
+//     read it) and the PCG vectors in the registers of the lanes that own them;
 //   * there is no barrier: every value that crosses CTAs travels as a 16-byte
 //     packet {double, tag} written and read in one 128-bit access, so the
 //     reader polls the datum itself and one L2 round trip carries both the
@@ -24,9 +25,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
+#include <cmath>
 #include <cstdint>
 #include <mutex>
 #include <numeric>
+#include <thread>
+#include <type_traits>
 
 #include "device_math.cuh"
 #include "engine.h"
@@ -45,27 +50,34 @@ constexpr int kRowThreads = kRowWarps * 32;
 // ten rows (a row never straddles a warp, so its w reaches m = Dinv w by
 // shuffles), in up to kMaxSets sets of kSetRows rows.
 constexpr int kSetRows = kRowWarps * 10;
-constexpr int kMaxSets = 2;
+constexpr int kMaxSets = 3;
 constexpr int kTeamMaxRows = kSetRows * kMaxSets;
-// blocks of a lane's first row that stay in its registers for the solve
-__host__ __device__ constexpr int reg_blocks(int sets) { return sets == 1 ? 3 : 1; }
-constexpr int kWantRows = 60, kAloneRows = 96;  // see plan_team
+// steps of a lane's first row group whose blocks stay in its registers
+__host__ __device__ constexpr int reg_blocks(int sets, bool dil) { return sets == 1 ? (dil ? 1 : 2) : 0; }
+constexpr int kWantRows = 46, kWantTeam = 80, kAloneRows = 96;  // see plan_team
+constexpr double kExchangeRows = 165, kSetupRows = 3000, kFill = 0.95;  // see plan_team
+constexpr int kRowWeight = 8;  // a row's vectors, in blocks
 constexpr int kTeamMaxRestarts = 10;  // as in pcg.cu
+// The recurrences run on to this part of the tolerance (2-3 per cent more
+// iterations), so that the true residual that decides meets it in the first
+// round in spite of their drift.
+constexpr double kStopShort = 0.6;
 constexpr int kTeamRoundCap = 400;    // as in pcg.cu
 
 struct TeamArgs {
   const TeamSlot* slots;
   int n_slots;
   unsigned long long* ticket;
-  const int* rows;         // slot-major: the global rows each slot owns (ascending)
-  const unsigned char* pub;  // per owned row (slot-major): some other CTA reads it
+  const int* rows;         // slot-major: the global rows each slot owns (most blocks first)
+  const unsigned char* pub;  // per owned row: some other CTA reads it
+  const int* diag;         // per owned row: its diagonal block in S
   const int* halo;         // slot-major: the global rows of other slots that the slot reads
-  const int* ro;           // slot-major, nloc + 1 per slot: block offsets within the slot
-  const int* src;          // per owned row: first block of the row in S
-  const unsigned short* dloc;  // per owned row: its diagonal block within the row
-  const unsigned short* cl;  // slot-major: per block its column as a local index (owned, then halo)
-  const int* g1;           // factored NODAL: per block the divBlk slots of d_row(col) and d_col(row) (-1 none)
+  const int4* group;       // slot-major: the row groups (RowGroup)
+  const int* blk;          // per step and lane: the block of S (-1: none)
+  const unsigned short* cl;  // per step and lane: its column as a local index (owned, then halo)
+  const int* g1;           // factored NODAL, per step and lane: divBlk slots of d_row(col) and d_col(row) (-1 none)
   const int* g2;
+  unsigned char* stream;   // steps beyond a slot's shared memory
   const void* S;
   const double* b;
   double* x;
@@ -140,34 +152,49 @@ struct PollBound {
   }
 };
 
+// Bytes of one step of a warp, value by value across the 32 lanes, so that its
+// loads are contiguous and free of bank conflicts: the lanes' blocks of S
+// (and, factored NODAL, d_row(col)), and d_col(row), which the product's second
+// half reads.
+__host__ __device__ constexpr int step_bytes(int mt_bytes, bool dil) { return 32 * (9 * mt_bytes + (dil ? 24 : 0)); }
+constexpr int kStep2 = 32 * 24;
 __host__ __device__ inline size_t team_align(size_t b) { return (b + 15) & ~(size_t)15; }
+// shared memory of one slot; the steps of S kept there come last
 struct TeamLayout {
-  size_t S, g, xs, sn, ts, ckp, ro, halo, cl, total;
+  size_t xs, sn, ts, ckp, halo, group, cl, G2, S;
 };
-__host__ __device__ inline TeamLayout team_layout(int nloc, int nb, int nh, int mt_bytes, bool dil) {
+__host__ __device__ inline TeamLayout team_layout(int nloc, int nh, int steps, int groups, bool dil) {
   TeamLayout o;
   size_t p = 0;
-  o.S = p;
-  p += team_align((size_t)nb * 9 * mt_bytes);
-  o.g = p;
-  if (dil) p += team_align((size_t)nb * 6 * sizeof(double));
+  o.group = p;
+  p += (size_t)groups * sizeof(int4);
   o.xs = p;
   p += team_align((size_t)(nloc + nh) * 3 * sizeof(double));
   o.sn = p;
-  p += team_align((size_t)nloc * 3 * sizeof(double));
+  p += team_align((size_t)nloc * (dil ? 6 : 3) * sizeof(double));
   o.ts = p;
   if (dil) p += team_align((size_t)(nloc + nh) * sizeof(double));
   o.ckp = p;
   if (dil) p += team_align((size_t)nloc * sizeof(double));
-  o.ro = p;
-  p += team_align((size_t)(nloc + 1) * sizeof(int));
   o.halo = p;
   p += team_align((size_t)nh * sizeof(int));
   o.cl = p;
-  p += team_align((size_t)nb * sizeof(unsigned short));
-  o.total = p;
+  p += team_align((size_t)steps * 32 * sizeof(unsigned short));
+  o.G2 = p;
+  if (dil) p += (size_t)steps * kStep2;
+  o.S = p;
   return o;
 }
+// A row group: the rows one warp walks together, 32 >> log lanes each of 1 << log
+struct RowGroup {
+  int shape;  // steps | log << 16 | (rows - 1) << 24
+  int step;   // its first step
+  int mem;    // its first step of S in memory (the register steps take none)
+  int row;    // its first local row
+  __device__ __forceinline__ int steps() const { return shape & 0xffff; }
+  __device__ __forceinline__ int log() const { return (shape >> 16) & 255; }
+  __device__ __forceinline__ int rows() const { return (shape >> 24) + 1; }
+};
 
 __device__ __forceinline__ void row_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kRowThreads) : "memory"); }
 
@@ -225,16 +252,17 @@ __global__ void team_state_kernel(int R, const int* __restrict__ act_node, const
   for (int c = 0; c < 3; c++) x[3 * (size_t)n + c] = xn[c];
 }
 
-// L: lanes per block row in the SpMV; SETS: component sets (rows <= SETS *
-// kSetRows); DIL: the factored NODAL matrix.
-template <typename MT, int L, int SETS, bool DIL>
+// SETS: component sets (rows <= SETS * kSetRows); DIL: the factored NODAL
+// matrix.
+template <typename MT, int SETS, bool DIL>
 __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ double s_part[kRowWarps][3];
   __shared__ double s_al, s_be;
   __shared__ int s_code, s_abort;
   __shared__ int s_ticket;
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, gl = lane & (L - 1);
+  __shared__ TeamSlot s_slot;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const bool red = warp == kRowWarps;
   // an error of an earlier launch of the call: nothing runs
   if (*(volatile int*)a.flags != 0) return;
@@ -248,7 +276,11 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
     const int si = s_ticket;
     __syncthreads();
     if (si >= a.n_slots) return;
-    const TeamSlot sl = a.slots[si];
+    // (in shared memory: the iterations need few of its fields, the registers
+    // are for the vectors and the matrix)
+    if (t == 0) s_slot = a.slots[si];
+    __syncthreads();
+    const TeamSlot& sl = s_slot;
     if (a.model_active && !a.model_active[sl.model]) {
       if (sl.rank == 0 && t == 0) {
         double* o = a.model_out + (size_t)sl.model * 4;
@@ -258,63 +290,47 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
       }
       continue;
     }
-    const int nloc = sl.nloc, nh = sl.nh, nb = sl.nb, k = sl.k;
+    const int nloc = sl.nloc, nh = sl.nh, k = sl.k;
     // tags continue from the model's last solve: a packet left by it never
     // carries a tag of this one
     const unsigned tag0 = a.base[sl.model];
     const double* sp = a.step + (size_t)sl.model * 8;
-    const TeamLayout lay = team_layout(nloc, nb, nh, (int)sizeof(MT), DIL);
-    MT* const S = (MT*)(dyn + lay.S);
-    double* const gs = (double*)(dyn + lay.g);  // per block d_row(col), d_col(row)
+    constexpr int kReg = reg_blocks(SETS, DIL), kStep = step_bytes((int)sizeof(MT), DIL);
+    const int ng = sl.groups;
+    const TeamLayout lay = team_layout(nloc, nh, sl.steps, ng, DIL);
     double* const xs = (double*)(dyn + lay.xs);
     double* const sn = (double*)(dyn + lay.sn);
     double* const ts = (double*)(dyn + lay.ts);
     double* const ckp = (double*)(dyn + lay.ckp);
-    int* const ro = (int*)(dyn + lay.ro);
     int* const hrow = (int*)(dyn + lay.halo);
+    RowGroup* const grp = (RowGroup*)(dyn + lay.group);
     unsigned short* const cl = (unsigned short*)(dyn + lay.cl);
+    unsigned char* const Ss = dyn + lay.S;
+    double* const g2s = (double*)(dyn + lay.G2);
+    unsigned char* const Sg = a.stream + (size_t)sl.stream0 * kStep;  // steps from sl.steps_smem on
+    // the warp's row group of a pass (alternating direction: the groups get
+    // shorter), -1 beyond the last
+    auto group_of = [&](int pass) {
+      const int g = pass * kRowWarps + ((pass & 1) ? kRowWarps - 1 - warp : warp);
+      return g < ng ? g : -1;
+    };
+    const int passes = (ng + kRowWarps - 1) / kRowWarps;
 
-    // ---- the slot's matrix, columns and starting vector to shared memory
-    for (int i = t; i <= nloc; i += kTeamThreads) ro[i] = a.ro[sl.ro0 + i];
+    // ---- the slot's tables and starting vector to shared memory
     for (int i = t; i < nh; i += kTeamThreads) hrow[i] = a.halo[sl.h0 + i];
-    for (int i = t; i < nb; i += kTeamThreads) cl[i] = a.cl[sl.b0 + i];
-    __syncthreads();
-    {
-      // a warp per row: the row's blocks are contiguous in S
-      const MT* Sg = (const MT*)a.S;
-      for (int i = warp; i < nloc; i += kTeamWarps) {
-        const int o = ro[i] * 9, n = ro[i + 1] * 9 - o;
-        const MT* sv = Sg + (size_t)a.src[sl.r0 + i] * 9;
-        for (int q = lane; q < n; q += 32) {
-          const unsigned d = (unsigned)__cvta_generic_to_shared(S + o + q);
-          asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(sv + q), "n"((int)sizeof(MT)));
-        }
-      }
-      asm volatile("cp.async.commit_group;");
-    }
+    for (int i = t; i < ng; i += kTeamThreads) ((int4*)grp)[i] = a.group[sl.g0 + i];
+    for (int i = t; i < sl.steps * 16; i += kTeamThreads)
+      ((unsigned*)cl)[i] = ((const unsigned*)(a.cl + (size_t)sl.w0 * 32))[i];
     for (int i = t; i < nloc + nh; i += kTeamThreads) {
-      const int r = i < nloc ? a.rows[sl.r0 + i] : hrow[i - nloc];
+      const int r = i < nloc ? a.rows[sl.r0 + i] : a.halo[sl.h0 + i - nloc];
 #pragma unroll
       for (int c = 0; c < 3; c++) xs[3 * i + c] = a.x[3 * (size_t)r + c];
-    }
-    if constexpr (DIL) {
-      for (int i = t; i < nb; i += kTeamThreads) {
-        const int q1 = a.g1[sl.b0 + i], q2 = a.g2[sl.b0 + i];
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-          gs[6 * i + c] = q1 >= 0 ? a.divblk[3 * (size_t)q1 + c] : 0.0;
-          gs[6 * i + 3 + c] = q2 >= 0 ? a.divblk[3 * (size_t)q2 + c] : 0.0;
-        }
-      }
-      const double cm = sp[0] * sp[0] + sp[0] * sp[2];
-      for (int i = t; i < nloc + nh; i += kTeamThreads) {
-        const int r = i < nloc ? a.rows[sl.r0 + i] : hrow[i - nloc];
-        const double v = cm * a.node_kp[a.act_node[r]];
+      if constexpr (DIL) {
+        const double v = (sp[0] * sp[0] + sp[0] * sp[2]) * a.node_kp[a.act_node[r]];
         ts[i] = v;  // until the first product: kp of the neighbours for the block diagonal
         if (i < nloc) ckp[i] = v;
       }
     }
-    asm volatile("cp.async.wait_group 0;");
     __syncthreads();
 
     if ((int)blockIdx.x == a.skip_cta) {
@@ -350,7 +366,8 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
         sums[1] = __shfl_sync(0xffffffffu, v, 8);
         sums[2] = __shfl_sync(0xffffffffu, v, 16);
         if (k > 1 && lane < 2)
-          put_packet(a.part_pk + ((size_t)(pe & 1) * a.n_slots + si) * 4 + 2 * lane, lane ? sums[1] : sums[0],
+          put_packet(a.part_pk + ((size_t)(pe & 1) * a.n_slots + sl.s0 + sl.rank) * 4 + 2 * lane,
+                     lane ? sums[1] : sums[0],
                      lane ? (unsigned)__double2loint(sums[2]) : (unsigned)__double2hiint(sums[2]), tag0 + pe + 1);
         pe++;
       };
@@ -358,13 +375,12 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
       // pairs take the two packets of a slot
       auto collect = [&]() {
         if (k == 1) return;
-        const double* buf = a.part_pk + (size_t)((pe - 1) & 1) * a.n_slots * 4 + 2 * (lane & 1);
+        const double* buf = a.part_pk + ((size_t)((pe - 1) & 1) * a.n_slots + sl.s0) * 4 + 2 * (lane & 1);
         const unsigned tag = tag0 + pe;
-        const int qe = sl.s0 + k;
         PollBound pb(a.flags, a.timeout_ns);
         double m = 0, r = 0;
-        constexpr int U = 5;
-        for (int qb = sl.s0; qb < qe; qb += 16 * U) {
+        auto round = [&](auto width, int qb) {
+          constexpr int U = decltype(width)::value;
           double v[U];
           unsigned hf[U];
           for (;;) {
@@ -374,7 +390,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
               const int q = qb + 16 * u + (lane >> 1);
               v[u] = 0;
               hf[u] = 0;
-              if (q < qe) {
+              if (q < k) {
                 unsigned g;
                 v[u] = get_packet(buf + (size_t)q * 4, hf[u], g);
                 all &= g == tag;
@@ -393,7 +409,11 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
             // (meaningful in the even lanes)
             r += __hiloint2double((int)hf[u], (int)o);
           }
-        }
+        };
+        if (k <= 16) round(std::integral_constant<int, 1>{}, 0);
+        else if (k <= 48) round(std::integral_constant<int, 3>{}, 0);
+        else
+          for (int qb = 0; qb < k; qb += 160) round(std::integral_constant<int, 10>{}, qb);
         if (lane & 1) r = 0;
 #pragma unroll
         for (int off = 16; off > 1; off >>= 1) {
@@ -411,7 +431,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
         if (have_bb) return;
         collect();
         bb = sums[0];
-        thr2 = tol * tol * bb;
+        thr2 = kStopShort * kStopShort * tol * tol * bb;
         have_bb = true;
       };
       __syncthreads();  // C of P0
@@ -569,67 +589,126 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
         }
         e++;
       };
-      // the lane's blocks of its first row in registers (double in both
-      // forms: the conversion is paid once per solve)
-      constexpr int kRegBlocks = reg_blocks(SETS);
-      double R[kRegBlocks][9];
-      int rc[kRegBlocks];
-      const int i0 = warp * (32 / L) + lane / L;  // first row of the lane's group
-      const int pr0 = i0 < nloc ? ro[i0] + gl : 0, pr1 = i0 < nloc ? ro[i0 + 1] : 0;
+      // The lane's blocks: the first kReg steps of its first row group in
+      // registers (double in both forms: the conversion is paid once per
+      // solve), the others in shared memory or in the slot's stream.
+      double R[kReg > 0 ? kReg : 1][9];
+      int rc[kReg > 0 ? kReg : 1];
+      const int g_first = group_of(0);
+      const int st_first = g_first >= 0 ? grp[g_first].steps() : 0;
 #pragma unroll
-      for (int b = 0; b < kRegBlocks; b++) {
-        const int p = pr0 + L * b;
-        const bool in = p < pr1;
-        rc[b] = in ? 3 * (int)cl[p] : 0;
+      for (int b = 0; b < kReg; b++) {
+        rc[b] = 0;
 #pragma unroll
-        for (int q = 0; q < 9; q++) R[b][q] = in ? (double)S[9 * p + q] : 0.0;
+        for (int v = 0; v < 9; v++) R[b][v] = 0;
+        if (b < st_first) {
+          const int at = (grp[g_first].step + b) * 32 + lane;
+          const int blk = a.blk[(size_t)sl.w0 * 32 + at];
+          rc[b] = 3 * (int)cl[at];
+          if (blk >= 0) {
+            const MT* B = (const MT*)a.S + 9 * (size_t)blk;
+#pragma unroll
+            for (int v = 0; v < 9; v++) R[b][v] = (double)B[v];
+          }
+        }
       }
+      for (int pass = 0; pass < passes; pass++) {
+        const int g = group_of(pass);
+        if (g < 0) continue;
+        const RowGroup rg = grp[g];
+        for (int b = 0; b < rg.steps(); b++) {
+          const size_t at = ((size_t)sl.w0 + rg.step + b) * 32 + lane;
+          if constexpr (DIL) {
+            const int q2 = a.g2[at];
+            double* gd = g2s + (size_t)(rg.step + b) * 96 + lane;
+#pragma unroll
+            for (int c = 0; c < 3; c++) gd[32 * c] = q2 >= 0 ? a.divblk[3 * (size_t)q2 + c] : 0.0;
+          }
+          // (register steps of the factored matrix keep d_row(col) in memory)
+          if (!DIL && pass == 0 && b < kReg) continue;
+          const int idx = rg.mem + b - (!DIL && pass == 0 ? kReg : 0);
+          unsigned char* dst = idx < sl.steps_smem ? Ss + (size_t)idx * kStep : Sg + (size_t)(idx - sl.steps_smem) * kStep;
+          const int blk = a.blk[at];
+          const MT* B = (const MT*)a.S + 9 * (size_t)max(blk, 0);
+#pragma unroll
+          for (int v = 0; v < 9; v++) ((MT*)dst)[32 * v + lane] = blk >= 0 ? B[v] : MT(0);
+          if constexpr (DIL) {
+            double* gd = (double*)(dst + 32 * 9 * sizeof(MT));
+            const int q1 = a.g1[at];
+#pragma unroll
+            for (int c = 0; c < 3; c++) gd[32 * c + lane] = q1 >= 0 ? a.divblk[3 * (size_t)q1 + c] : 0.0;
+          }
+        }
+      }
+      // one step of a row group from memory
+      auto add_step = [&](const unsigned char* src, int c, bool with_S, double& a0, double& a1, double& a2, double& tt) {
+        const double* xv = xs + 3 * c;
+        const double x0 = xv[0], x1 = xv[1], x2 = xv[2];
+        const MT* B = (const MT*)src + lane;
+        if (with_S) {
+          a0 += (double)B[0] * x0 + (double)B[32] * x1 + (double)B[64] * x2;
+          a1 += (double)B[96] * x0 + (double)B[128] * x1 + (double)B[160] * x2;
+          a2 += (double)B[192] * x0 + (double)B[224] * x1 + (double)B[256] * x2;
+        }
+        if constexpr (DIL) {
+          const double* gd = (const double*)(src + 32 * 9 * sizeof(MT)) + lane;
+          tt += gd[0] * x0 + gd[32] * x1 + gd[64] * x2;
+        }
+      };
+      // steps in flight at once: memory-bound slots want more, the small ones
+      // their registers for the matrix
+      constexpr int kFlight = SETS == 1 ? 1 : 2;
       // sn = S xs for the slot's rows (xs complete behind the row barrier)
       auto product = [&]() {
         row_barrier();
-        constexpr int G = 32 / L;
-        for (int base = warp * G, pass = 0; base < nloc; base += kRowWarps * G, pass++) {
-          const int i = base + lane / L;
-          const bool valid = i < nloc;
+#pragma unroll 1
+        for (int pass = 0; pass < passes; pass++) {
+          const int g = group_of(pass);
+          if (g < 0) continue;
+          const RowGroup rg = grp[g];
+          const int st = rg.steps();
+          const unsigned short* cp = cl + rg.step * 32 + lane;
+          int idx = rg.mem, b = 0;
           double a0 = 0, a1 = 0, a2 = 0, tt = 0;
-          int p = 0, p1 = 0;
-          if (pass == 0) {
+          if (kReg > 0 && pass == 0) {
 #pragma unroll
-            for (int b = 0; b < kRegBlocks; b++) {
-              const double* xv = xs + rc[b];
+            for (int q = 0; q < kReg; q++) {
+              const double* xv = xs + rc[q];
               const double x0 = xv[0], x1 = xv[1], x2 = xv[2];
-              a0 += R[b][0] * x0 + R[b][1] * x1 + R[b][2] * x2;
-              a1 += R[b][3] * x0 + R[b][4] * x1 + R[b][5] * x2;
-              a2 += R[b][6] * x0 + R[b][7] * x1 + R[b][8] * x2;
+              a0 += R[q][0] * x0 + R[q][1] * x1 + R[q][2] * x2;
+              a1 += R[q][3] * x0 + R[q][4] * x1 + R[q][5] * x2;
+              a2 += R[q][6] * x0 + R[q][7] * x1 + R[q][8] * x2;
               if constexpr (DIL) {
-                const int pp = pr0 + L * b;
-                if (pp < pr1) tt += gs[6 * pp] * x0 + gs[6 * pp + 1] * x1 + gs[6 * pp + 2] * x2;
+                if (q < st) {
+                  const unsigned char* src = idx + q < sl.steps_smem ? Ss + (size_t)(idx + q) * kStep
+                                                                    : Sg + (size_t)(idx + q - sl.steps_smem) * kStep;
+                  const double* gd = (const double*)(src + 32 * 9 * sizeof(MT)) + lane;
+                  tt += gd[0] * x0 + gd[32] * x1 + gd[64] * x2;
+                }
               }
             }
-            p = pr0 + L * kRegBlocks;
-            p1 = pr1;
-          } else if (valid) {
-            p = ro[i] + gl;
-            p1 = ro[i + 1];
+            b = kReg;
+            if (DIL) idx += kReg;
           }
-#pragma unroll 1
-          for (; p < p1; p += L) {
-            const double* xv = xs + 3 * (int)cl[p];
-            const MT* B = S + 9 * p;
-            const double x0 = xv[0], x1 = xv[1], x2 = xv[2];
-            a0 += (double)B[0] * x0 + (double)B[1] * x1 + (double)B[2] * x2;
-            a1 += (double)B[3] * x0 + (double)B[4] * x1 + (double)B[5] * x2;
-            a2 += (double)B[6] * x0 + (double)B[7] * x1 + (double)B[8] * x2;
-            if constexpr (DIL) tt += gs[6 * p] * x0 + gs[6 * p + 1] * x1 + gs[6 * p + 2] * x2;
+          const int in_smem = min(st - b, sl.steps_smem - idx);
+#pragma unroll kFlight
+          for (int q = 0; q < in_smem; q++) add_step(Ss + (size_t)(idx + q) * kStep, cp[32 * (b + q)], true, a0, a1, a2, tt);
+          const int done = max(in_smem, 0);
+          const unsigned char* sg = Sg + (ptrdiff_t)(idx + done - sl.steps_smem) * kStep;
+#pragma unroll kFlight
+          for (int q = done; q < st - b; q++) {
+            add_step(sg, cp[32 * (b + q)], true, a0, a1, a2, tt);
+            sg += kStep;
           }
-#pragma unroll
-          for (int off = L / 2; off > 0; off >>= 1) {
+          for (int off = (1 << rg.log()) >> 1; off > 0; off >>= 1) {
             a0 += __shfl_xor_sync(0xffffffffu, a0, off);
             a1 += __shfl_xor_sync(0xffffffffu, a1, off);
             a2 += __shfl_xor_sync(0xffffffffu, a2, off);
             if constexpr (DIL) tt += __shfl_xor_sync(0xffffffffu, tt, off);
           }
-          if (valid && gl == 0) {
+          const int sub = lane >> rg.log();
+          if ((lane & ((1 << rg.log()) - 1)) == 0 && sub < rg.rows()) {
+            const int i = rg.row + sub;
             sn[3 * i] = a0;
             sn[3 * i + 1] = a1;
             sn[3 * i + 2] = a2;
@@ -663,29 +742,30 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
           }
           te++;
           row_barrier();
-          for (int base = warp * G; base < nloc; base += kRowWarps * G) {
-            const int i = base + lane / L;
-            const bool valid = i < nloc;
-            int p = 0, p1 = 0;
-            if (valid) {
-              p = ro[i] + gl;
-              p1 = ro[i + 1];
-            }
+#pragma unroll 1
+          for (int pass = 0; pass < passes; pass++) {
+            const int g = group_of(pass);
+            if (g < 0) continue;
+            const RowGroup rg = grp[g];
+            const int st = rg.steps();
+            const unsigned short* cp = cl + rg.step * 32 + lane;
+            const double* gd = g2s + (size_t)rg.step * 96 + lane;
             double a0 = 0, a1 = 0, a2 = 0;
 #pragma unroll 2
-            for (; p < p1; p += L) {
-              const double tv = ts[cl[p]];
-              a0 += tv * gs[6 * p + 3];
-              a1 += tv * gs[6 * p + 4];
-              a2 += tv * gs[6 * p + 5];
+            for (int b = 0; b < st; b++) {
+              const double tv = ts[cp[32 * b]];
+              a0 += tv * gd[96 * b];
+              a1 += tv * gd[96 * b + 32];
+              a2 += tv * gd[96 * b + 64];
             }
-#pragma unroll
-            for (int off = L / 2; off > 0; off >>= 1) {
+            for (int off = (1 << rg.log()) >> 1; off > 0; off >>= 1) {
               a0 += __shfl_xor_sync(0xffffffffu, a0, off);
               a1 += __shfl_xor_sync(0xffffffffu, a1, off);
               a2 += __shfl_xor_sync(0xffffffffu, a2, off);
             }
-            if (valid && gl == 0) {
+            const int sub = lane >> rg.log();
+            if ((lane & ((1 << rg.log()) - 1)) == 0 && sub < rg.rows()) {
+              const int i = rg.row + sub;
               sn[3 * i] += a0;
               sn[3 * i + 1] += a1;
               sn[3 * i + 2] += a2;
@@ -725,13 +805,42 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
         D[j][0] = D[j][1] = D[j][2] = 0;
       }
 
+      if constexpr (DIL) {
+        // the dilational term's diagonal blocks, sum_n c kp_n d_n(row) d_n(row)^T
+        // (their six different entries), into sn
+        for (int pass = 0; pass < passes; pass++) {
+          const int g = group_of(pass);
+          if (g < 0) continue;
+          const RowGroup rg = grp[g];
+          const unsigned short* cp = cl + rg.step * 32 + lane;
+          const double* gd = g2s + (size_t)rg.step * 96 + lane;
+          double q6[6] = {0, 0, 0, 0, 0, 0};
+          for (int b = 0; b < rg.steps(); b++) {
+            const double ck = ts[cp[32 * b]], y0 = gd[96 * b], y1 = gd[96 * b + 32], y2 = gd[96 * b + 64];
+            q6[0] += ck * y0 * y0;
+            q6[1] += ck * y0 * y1;
+            q6[2] += ck * y0 * y2;
+            q6[3] += ck * y1 * y1;
+            q6[4] += ck * y1 * y2;
+            q6[5] += ck * y2 * y2;
+          }
+          for (int off = (1 << rg.log()) >> 1; off > 0; off >>= 1)
+#pragma unroll
+            for (int c = 0; c < 6; c++) q6[c] += __shfl_xor_sync(0xffffffffu, q6[c], off);
+          const int sub = lane >> rg.log();
+          if ((lane & ((1 << rg.log()) - 1)) == 0 && sub < rg.rows())
+#pragma unroll
+            for (int c = 0; c < 6; c++) sn[6 * (rg.row + sub) + c] = q6[c];
+        }
+        row_barrier();
+      }
       // ---- P0: block-Jacobi inverse, r = b - S x0, u = Dinv r; ||b||^2,
       // r.u, r.r
 #pragma unroll
       for (int j = 0; j < SETS; j++) {
         if (oi[j] < 0) continue;
         const int i = oi[j];
-        const MT* B = S + 9 * (ro[i] + a.dloc[sl.r0 + i]);
+        const MT* B = (const MT*)a.S + 9 * (size_t)a.diag[sl.r0 + i];
         double dg[9], inv[9];
 #pragma unroll
         for (int c = 0; c < 9; c++) {
@@ -739,15 +848,16 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
           inv[c] = 0;
         }
         if constexpr (DIL) {
-          // the dilational term's diagonal block: sum_n c kp_n d_n(row) d_n(row)^T
-          for (int pb = ro[i]; pb < ro[i + 1]; pb++) {
-            const double* g = gs + 6 * pb + 3;
-            const double ck = ts[cl[pb]];
-#pragma unroll
-            for (int m = 0; m < 3; m++)
-#pragma unroll
-              for (int l = 0; l < 3; l++) dg[3 * m + l] += ck * g[m] * g[l];
-          }
+          const double* q6 = sn + 6 * i;
+          dg[0] += q6[0];
+          dg[1] += q6[1];
+          dg[2] += q6[2];
+          dg[3] += q6[1];
+          dg[4] += q6[3];
+          dg[5] += q6[4];
+          dg[6] += q6[2];
+          dg[7] += q6[4];
+          dg[8] += q6[5];
         }
         if (invert3(inv, dg) == 0.0) {
           // a singular diagonal block: the solve ends at the next barrier B
@@ -772,7 +882,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
 #pragma unroll
         for (int c = 0; c < 3; c++) D[j][c] = oc == 0 ? inv[c] : oc == 1 ? inv[3 + c] : inv[6 + c];
       }
-      product();      // (its first barrier also ends the reads of kp in ts)
+      product();      // (its first barrier also ends the reads of kp in ts and of sn)
       row_barrier();  // sn
       double d0 = 0, d1 = 0, d2 = 0;
       {
@@ -969,45 +1079,69 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
 
 using TeamKernel = void (*)(TeamArgs);
 template <typename MT, bool DIL>
-TeamKernel team_kernel_of(int lanes, int sets) {
-  if (sets > 1) return lanes == 4 ? pcg_team_kernel<MT, 4, 2, DIL> : pcg_team_kernel<MT, 8, 2, DIL>;
-  return lanes == 4 ? pcg_team_kernel<MT, 4, 1, DIL> : lanes == 8 ? pcg_team_kernel<MT, 8, 1, DIL>
-                                                                   : pcg_team_kernel<MT, 16, 1, DIL>;
+TeamKernel team_kernel_of(int sets) {
+  return sets == 3 ? pcg_team_kernel<MT, 3, DIL> : sets == 2 ? pcg_team_kernel<MT, 2, DIL> : pcg_team_kernel<MT, 1, DIL>;
 }
 TeamKernel team_kernel(const Engine& eng) {
   const bool dil = eng.factored && eng.d.n_dil_nodes > 0;
   if (eng.precision == B200FEM_PREC_MIXED)
-    return dil ? team_kernel_of<float, true>(eng.team_lanes, eng.team_sets)
-               : team_kernel_of<float, false>(eng.team_lanes, eng.team_sets);
-  return dil ? team_kernel_of<double, true>(eng.team_lanes, eng.team_sets)
-             : team_kernel_of<double, false>(eng.team_lanes, eng.team_sets);
+    return dil ? team_kernel_of<float, true>(eng.team_sets) : team_kernel_of<float, false>(eng.team_sets);
+  return dil ? team_kernel_of<double, true>(eng.team_sets) : team_kernel_of<double, false>(eng.team_sets);
 }
 
-// Recursive bisection of `rows` into k parts of nearly equal size along the
-// longest axis of their nodes' rest positions; part[i] of the i-th row.
-void bisect(std::vector<int>& rows, int a, int b, int k, const double* pos, const int* node, std::vector<int>& cut) {
+// f(thread, i) for i in [0, n) on up to `threads` host threads.
+template <typename F>
+void parallel_for(int n, int threads, F&& f) {
+  std::atomic<int> next(0);
+  auto work = [&](int th) {
+    for (int i; (i = next++) < n;) f(th, i);
+  };
+  std::vector<std::thread> pool;
+  for (int th = 1; th < std::min(threads, n); th++) pool.emplace_back(work, th);
+  work(0);
+  for (auto& t : pool) t.join();
+}
+int host_threads() { return (int)std::min(16u, std::max(1u, std::thread::hardware_concurrency())); }
+
+// Recursive bisection of rows [a, b) into k parts of nearly equal weight along
+// the longest axis of their nodes' rest positions.
+// The cuts go to cut[0 .. k - 1]; the two halves of a large range are cut in
+// parallel.
+void bisect(std::vector<int>& rows, int a, int b, int k, const double* pos, const int* node,
+            const std::vector<int>& weight, int* cut) {
   if (k <= 1) {
-    cut.push_back(b);
+    cut[0] = b;
     return;
   }
   double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-  for (int i = a; i < b; i++)
+  long long total = 0;
+  for (int i = a; i < b; i++) {
+    total += weight[rows[i]];
     for (int c = 0; c < 3; c++) {
       const double v = pos[3 * (size_t)node[rows[i]] + c];
       lo[c] = std::min(lo[c], v);
       hi[c] = std::max(hi[c], v);
     }
+  }
   int ax = 0;
   for (int c = 1; c < 3; c++)
     if (hi[c] - lo[c] > (hi[ax] - lo[ax]) * (1 + 1e-9)) ax = c;
+  std::vector<std::pair<double, int>> key(b - a);
+  for (int i = a; i < b; i++) key[i - a] = {pos[3 * (size_t)node[rows[i]] + ax], rows[i]};
+  std::sort(key.begin(), key.end());
+  for (int i = a; i < b; i++) rows[i] = key[i - a].second;
   const int kl = k / 2;
-  const int mid = a + (int)((long long)(b - a) * kl / k);
-  std::nth_element(rows.begin() + a, rows.begin() + mid, rows.begin() + b, [&](int x, int y) {
-    const double px = pos[3 * (size_t)node[x] + ax], py = pos[3 * (size_t)node[y] + ax];
-    return px != py ? px < py : x < y;
-  });
-  bisect(rows, a, mid, kl, pos, node, cut);
-  bisect(rows, mid, b, k - kl, pos, node, cut);
+  long long sum = 0;
+  int mid = a;
+  // (every part keeps at least one row)
+  while (mid < b - (k - kl) && (mid < a + kl || (2 * sum + weight[rows[mid]]) * k <= 2 * total * kl))
+    sum += weight[rows[mid++]];
+  auto left = [&]() { bisect(rows, a, mid, kl, pos, node, weight, cut); };
+  std::thread other;
+  if (b - a >= 8192) other = std::thread(left);
+  else left();
+  bisect(rows, mid, b, k - kl, pos, node, weight, cut + kl);
+  if (other.joinable()) other.join();
 }
 
 }  // namespace
@@ -1016,11 +1150,12 @@ namespace {
 // One model's split over k CTAs (slot offsets relative to it)
 struct TeamSplit {
   std::vector<TeamSlot> slots;
-  std::vector<int> rows, ro, halo, blk;
+  std::vector<int> rows, halo, blk;
+  std::vector<int4> group;
   std::vector<unsigned short> cl;
   std::vector<unsigned char> pub;  // per row of the model
-  int nloc_max = 0;
   size_t smem = 0;
+  int stream = 0;
 };
 }  // namespace
 
@@ -1031,81 +1166,215 @@ static size_t team_smem_budget(int device) {
   return (size_t)std::max(0, optin - 2048);
 }
 
-// Splits one model's rows (rowptr/col: its pattern with global rows, blocks
-// counted from the pack's first) over k CTAs.  pos: node positions, node:
-// row - row0 -> node.  Returns false when a CTA would not fit.
-static bool team_split_model(int row0, int n, int k, const std::vector<int>& rowptr, const std::vector<int>& col,
-                      const double* pos, const int* node, int mt_bytes, bool dil, size_t budget, TeamSplit& out) {
-  std::vector<int> rows(n);
+// Adds the slots of `p` behind those of `out`.
+template <typename Dst>
+static void append_split(Dst& out, const TeamSplit& p) {
+  for (TeamSlot s : p.slots) {
+    s.r0 += (int)out.rows.size();
+    s.h0 += (int)out.halo.size();
+    s.g0 += (int)out.group.size();
+    s.w0 += (int)(out.cl.size() / 32);
+    s.stream0 += out.stream;
+    out.slots.push_back(s);
+  }
+  out.stream += p.stream;
+  out.smem = std::max(out.smem, p.smem);
+  out.rows.insert(out.rows.end(), p.rows.begin(), p.rows.end());
+  out.halo.insert(out.halo.end(), p.halo.begin(), p.halo.end());
+  out.group.insert(out.group.end(), p.group.begin(), p.group.end());
+  out.cl.insert(out.cl.end(), p.cl.begin(), p.cl.end());
+  out.blk.insert(out.blk.end(), p.blk.begin(), p.blk.end());
+}
+
+// Lanes (as a power of two) that walk a row of n blocks in at most T steps.
+static int lanes_log(int n, int T) {
+  int l = 1;
+  while (l < 5 && (T << l) < n) l++;
+  return l;
+}
+
+// Splits one model's n rows from row0 on (rowptr/col: the pattern with global
+// rows) over k CTAs of nearly equal weight.  pos: node positions, node: row -
+// row0 -> node.  A CTA's rows are ordered by their number of blocks, most
+// first, and a warp's row group holds rows with the same number of lanes,
+// chosen so that every row takes at most T steps; T is the smallest number
+// for which the groups are walked in one pass of the row warps (a latency:
+// the longest rows, 27 blocks in a tet mesh and over 60 in a quadratic one,
+// would otherwise hold up all others), or kManySteps where one pass cannot
+// do, which wastes few lanes.  A row's blocks are dealt to its steps and
+// lanes so that the sixteen lanes of a half-warp read x from different banks
+// where that can be had.  Steps of S that do not fit the shared memory are
+// streamed when `stream` allows it, else the split fails.
+constexpr int kManySteps = 6;
+static bool team_split_model(int row0, int n, int k, int sets, const std::vector<int>& rowptr,
+                             const std::vector<int>& col, const double* pos, const int* node, int mt_bytes, bool dil,
+                             size_t budget, bool stream, int threads, TeamSplit& result) {
+  std::vector<int> rows(n), cut(k), weight(n);
   std::iota(rows.begin(), rows.end(), 0);
-  std::vector<int> cut;
-  bisect(rows, 0, n, k, pos, node, cut);
-  out = TeamSplit();
-  std::vector<int> stamp(n, -1), loc(n, 0);
-  out.pub.assign(n, 0);
-  int a = 0;
-  for (int c = 0; c < k; c++) {
-    const int b = cut[c];
-    if (b <= a || b - a > kTeamMaxRows) return false;
-    std::sort(rows.begin() + a, rows.begin() + b);
+  auto len = [&](int r) { return rowptr[row0 + r + 1] - rowptr[row0 + r]; };
+  for (int r = 0; r < n; r++) weight[r] = len(r) + kRowWeight;
+  bisect(rows, 0, n, k, pos, node, weight, cut.data());
+  int nmax = 0;
+  for (int c = 0; c < k; c++) nmax = std::max(nmax, cut[c] - (c ? cut[c - 1] : 0));
+  if (nmax > sets * kSetRows) return false;
+  // register steps take no memory (the factored matrix keeps d_row(col) of
+  // all its steps there)
+  const int reg = dil ? 0 : reg_blocks(sets, false);
+  struct Scratch {
+    std::vector<int> stamp, loc, rem;
+  };
+  std::vector<Scratch> scratch(threads);
+  std::vector<TeamSplit> piece(k);
+  std::atomic<bool> fits(true);
+  // one CTA's slot; false when it does not fit
+  auto split_slot = [&](int th, int c) -> bool {
+    TeamSplit& out = piece[c];
+    std::vector<int>&stamp = scratch[th].stamp, &loc = scratch[th].loc, &rem = scratch[th].rem;
+    if (stamp.empty()) {
+      stamp.assign(n, -1);
+      loc.assign(n, 0);
+    }
+    const int a = c ? cut[c - 1] : 0, b = cut[c], nloc = b - a;
+    if (nloc <= 0) return false;
+    std::sort(rows.begin() + a, rows.begin() + b, [&](int x, int y) {
+      return len(x) != len(y) ? len(x) > len(y) : x < y;
+    });
     for (int i = a; i < b; i++) {
       stamp[rows[i]] = c;
       loc[rows[i]] = i - a;
     }
-    std::vector<int> halo;
-    int nb = 0;
-    for (int i = a; i < b; i++) {
-      const int r = row0 + rows[i];
-      nb += rowptr[r + 1] - rowptr[r];
-      for (int p = rowptr[r]; p < rowptr[r + 1]; p++) {
+    const int h0 = 0;
+    for (int i = a; i < b; i++)
+      for (int p = rowptr[row0 + rows[i]]; p < rowptr[row0 + rows[i] + 1]; p++) {
         const int j = col[p] - row0;
         if (stamp[j] != c) {
           stamp[j] = c;
-          halo.push_back(j);
+          out.halo.push_back(j);
         }
       }
-    }
-    std::sort(halo.begin(), halo.end());
-    const int nloc = b - a, nh = (int)halo.size();
-    if (nloc + nh > 65535 || team_layout(nloc, nb, nh, mt_bytes, dil).total > budget) return false;
+    std::sort(out.halo.begin() + h0, out.halo.end());
+    const int nh = (int)out.halo.size() - h0;
+    if (nloc + nh > 65535) return false;
     for (int h = 0; h < nh; h++) {
-      loc[halo[h]] = nloc + h;
-      out.pub[halo[h]] = 1;
+      loc[out.halo[h0 + h]] = nloc + h;
+      out.halo[h0 + h] += row0;
     }
     TeamSlot s{};
     s.rank = c;
     s.k = k;
     s.nloc = nloc;
     s.nh = nh;
-    s.nb = nb;
-    s.r0 = (int)out.rows.size();
-    s.ro0 = (int)out.ro.size();
-    s.h0 = (int)out.halo.size();
-    s.b0 = (int)out.cl.size();
-    int o = 0;
-    for (int i = a; i < b; i++) {
-      const int r = row0 + rows[i];
-      out.rows.push_back(r);
-      out.ro.push_back(o);
-      for (int p = rowptr[r]; p < rowptr[r + 1]; p++) {
-        out.cl.push_back((unsigned short)loc[col[p] - row0]);
-        out.blk.push_back(p);
+    for (int i = a; i < b; i++) out.rows.push_back(row0 + rows[i]);
+    auto count_groups = [&](int T) {
+      int g = 0;
+      for (int i = a; i < b; g++) i += 32 >> lanes_log(len(rows[i]), T);
+      return g;
+    };
+    int T = 1;
+    while (T <= 64 && count_groups(T) > kRowWarps) T++;
+    if (T > kManySteps && count_groups(kManySteps) > kRowWarps) T = std::min(T, kManySteps);
+    int mem = 0;  // steps of S kept in memory
+    for (int i1 = a; i1 < b;) {
+      const int lg = lanes_log(len(rows[i1]), T), L = 1 << lg;
+      const int g0 = i1, g1 = std::min(b, i1 + (32 >> lg));
+      const int steps = (len(rows[g0]) + L - 1) / L;
+      if (steps > 0xffff) return false;
+      out.group.push_back(int4{steps | lg << 16 | (g1 - g0 - 1) << 24, s.steps, mem, g0 - a});
+      mem += s.groups < kRowWarps ? std::max(0, steps - reg) : steps;
+      s.groups++;
+      const size_t at = out.cl.size();
+      out.cl.resize(at + 32 * (size_t)steps, 0);
+      out.blk.resize(at + 32 * (size_t)steps, -1);
+      const int half = std::max(1, 16 >> lg);
+      for (int i0 = g0; i0 < g1; i0 += half) {
+        const int nr = std::min(half, g1 - i0);
+        // the rows' blocks not placed yet, one list after the other
+        int start[16], left[16];
+        rem.clear();
+        for (int q = 0; q < nr; q++) {
+          start[q] = (int)rem.size();
+          const int r = row0 + rows[i0 + q];
+          for (int p = rowptr[r]; p < rowptr[r + 1]; p++) rem.push_back(p);
+          left[q] = (int)rem.size() - start[q];
+        }
+        for (int st = 0; st < steps; st++) {
+          unsigned char used[16] = {0};
+          int pad = 0;
+          for (int q = 0; q < nr; q++) {
+            for (int l = 0; l < L && left[q] > 0; l++) {
+              int best = 0, bu = 255;
+              for (int z = 0; z < left[q]; z++) {
+                const int u = used[loc[col[rem[start[q] + z]] - row0] & 15];
+                if (u < bu) {
+                  bu = u;
+                  best = z;
+                  if (u == 0) break;
+                }
+              }
+              const int p = rem[start[q] + best];
+              rem[start[q] + best] = rem[start[q] + --left[q]];
+              const int lc = loc[col[p] - row0];
+              used[lc & 15]++;
+              pad = lc;
+              const size_t w = at + 32 * (size_t)st + (size_t)(i0 - g0 + q) * L + l;
+              out.cl[w] = (unsigned short)lc;
+              out.blk[w] = p;
+            }
+          }
+          // lanes without a block read an address the half-warp reads anyway
+          for (int q = 0; q < nr * L; q++) {
+            const size_t w = at + 32 * (size_t)st + (size_t)(i0 - g0) * L + q;
+            if (out.blk[w] < 0) out.cl[w] = (unsigned short)pad;
+          }
+        }
       }
-      o += rowptr[r + 1] - rowptr[r];
+      s.steps += steps;
+      i1 = g1;
     }
-    out.ro.push_back(o);
-    for (int h : halo) out.halo.push_back(row0 + h);
+    const size_t fixed = team_layout(nloc, nh, s.steps, s.groups, dil).S;
+    if (fixed > budget) return false;
+    const size_t sb = step_bytes(mt_bytes, dil);
+    s.steps_smem = (int)std::min<size_t>(mem, (budget - fixed) / sb);
+    out.stream = mem - s.steps_smem;
+    if (!stream && s.steps_smem < mem) return false;
+    out.smem = fixed + sb * s.steps_smem;
     out.slots.push_back(s);
-    out.nloc_max = std::max(out.nloc_max, nloc);
-    out.smem = std::max(out.smem, team_layout(nloc, nb, nh, mt_bytes, dil).total);
-    a = b;
+    return true;
+  };
+  parallel_for(k, threads, [&](int th, int c) {
+    if (fits && !split_slot(th, c)) fits = false;
+  });
+  if (!fits) return false;
+  result = TeamSplit();
+  result.pub.assign(n, 0);
+  for (TeamSplit& p : piece) {
+    for (int h : p.halo) result.pub[h - row0] = 1;
+    append_split(result, p);
   }
   return true;
 }
 
+// A model's PCG iterations relative to other models', for the queue order
+// only: block-Jacobi PCG takes about sqrt(1 + h^2 w^2) of them, w = sqrt(M /
+// rho) / dx the highest frequency of the mesh (M the P-wave modulus).  The
+// step size is not known when the pack is built; h = 0.01 weighs stiff models
+// against soft ones.  Fitted to 700 uneven NeoHookean beams (5 to 590
+// iterations, correlation 0.97).
+static double expected_iterations(const ModelDesc& m, const ModelHost& h) {
+  const double* p = m.mat_params;
+  double modulus = 0;
+  if (m.mat_kind == B200FEM_MAT_MOONEYRIVLIN) modulus = p[5] + 8.0 / 3.0 * (p[0] + p[1]);
+  else modulus = p[0] * (1 - p[1]) / ((1 + p[1]) * (1 - 2 * p[1]));
+  double vol = 0;
+  for (double v : h.rest_vol) vol += v;
+  const double dx = std::cbrt(std::max(vol, 1e-300) / std::max(m.n_nodes, 1));
+  const double w = std::sqrt(std::max(modulus, 0.0) / std::max(m.density, 1e-300)) / dx;
+  const double it = 4 + 24 * 0.01 * w;
+  return std::isfinite(it) ? std::min(it, 1e6) : 4;
+}
+
 // The team layout of a pack: per model the number of CTAs, its split, and the
-// slots of all models in queue order (most rows first, so that the longest
-// solves start first and the short ones fill the CTAs they free).
+// slots of all models in queue order.
 bool plan_team(Engine& eng, int grid_max, const std::vector<int>& rowptr, const std::vector<int>& col,
                const std::vector<int>& diag, bool dil, TeamHost& out) {
   const int M = (int)eng.hosts.size();
@@ -1113,71 +1382,134 @@ bool plan_team(Engine& eng, int grid_max, const std::vector<int>& rowptr, const 
   const size_t budget = team_smem_budget(eng.device);
   const int R = eng.row_off[M];
   if (R <= 0 || grid_max <= 0) return false;
+  for (int r = 0; r < R; r++)  // a row without blocks (an active node in no element) has no diagonal
+    if (diag[r] < rowptr[r] || diag[r] >= rowptr[r + 1]) return false;
   // Rows per CTA wanted: all CTAs busy from the start, at least kWantRows.
-  // 60 rows give each row eight of the 480 row lanes; fewer rows per CTA put
-  // more CTAs into every sum (40x10x10 hex beam, us per iteration: 3.4 at 32
-  // rows in 148 CTAs, 2.8 at 64 rows in 76, 3.1 at 96; 1,958-row quadratic
-  // beam 2.9 at 32 rows, 3.0 at 48, 4.7 at 64, where four lanes walk its
-  // 23-block rows).  Up to kAloneRows one CTA needs no exchange at all: a
-  // 72-row beam 1.36 us per iteration against 1.6 in two CTAs.
-  const int want = std::max(kWantRows, (R + grid_max - 1) / grid_max);
-  std::vector<int> order;
+  // Fewer rows shorten the product and put more CTAs into every exchange (us
+  // per iteration: 40x10x10 hex beam 4.2 at 30 rows, 3.2 at 44, 3.3 at 60, 3.9
+  // at 90; 1,958-row quadratic beam 2.7, 2.2, 2.4, 3.5; 2,376-row NODAL block,
+  // whose two exchanges bound it, 4.3 at 12 to 60).  Up to kAloneRows one CTA
+  // needs no exchange at all: a 90-row beam 1.36 against 1.44 in two CTAs.
+  struct Range {
+    int lo, hi;   // fewest CTAs that hold the model's rows, most that help it
+    double it;
+  };
+  std::vector<int> order, team(M, 0);
   for (int m = 0; m < M; m++)
     if (eng.row_off[m + 1] > eng.row_off[m]) order.push_back(m);
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-    return eng.row_off[x + 1] - eng.row_off[x] > eng.row_off[y + 1] - eng.row_off[y];
+  // duration of one solve in the time of a row: the iterations' exchange and
+  // rows, and the slot's set-up (measured: 1.4 us per iteration and 8.5 ns per
+  // row of it, 26 us per slot)
+  auto cost = [&](const Range& r, int n, int k) { return r.it * (kExchangeRows + (double)n / k) + kSetupRows; };
+  auto plan = [&](int sets, std::vector<int>& teams) {
+    std::vector<Range> range(M);
+    double lo = 0, hi = 0;
+    for (int m : order) {
+      const int a = eng.row_off[m], n = eng.row_off[m + 1] - a;
+      const size_t need = (size_t)(rowptr[a + n] - rowptr[a]) * (9 * mt + 2 + (dil ? 48 : 0)) + (size_t)n * 48;
+      const int rows = sets * kSetRows * 8 / 9;  // parts of equal weight differ in their rows
+      Range& r = range[m];
+      r.lo = std::max({1, (int)((need + budget - 1) / budget), (n + rows - 1) / rows});
+      // beyond kWantTeam CTAs only rows count (the hex beam above)
+      r.hi = n <= kAloneRows ? 1
+                             : std::max(std::min((n + kWantRows - 1) / kWantRows, kWantTeam), n / (2 * kWantRows));
+      r.lo = std::min({r.lo, grid_max, n});
+      r.hi = std::max(r.lo, std::min(r.hi, grid_max));
+      r.it = expected_iterations(eng.models[m], eng.hosts[m]);
+      lo = std::max(lo, cost(r, n, r.hi));
+      hi += cost(r, n, r.lo) * r.lo;
+    }
+    // the shortest makespan that the CTAs' time allows: every model takes the
+    // fewest CTAs that end it in time (48 uneven beams, whose slowest holds
+    // three CTAs for 1.75 ms at their fewest, then end at 0.72 ms)
+    auto teams_for = [&](double T) {
+      double area = 0;
+      for (int m : order) {
+        const int n = eng.row_off[m + 1] - eng.row_off[m];
+        const Range& r = range[m];
+        int k = r.lo;
+        while (k < r.hi && cost(r, n, k) > T) k++;
+        teams[m] = k;
+        area += k * cost(r, n, k);
+      }
+      return area;
+    };
+    hi = std::max(hi, lo);
+    if (teams_for(lo) > kFill * grid_max * lo) {
+      for (int i = 0; i < 40; i++) {
+        const double T = 0.5 * (lo + hi);
+        if (teams_for(T) > kFill * grid_max * T) lo = T;
+        else hi = T;
+      }
+      teams_for(hi);
+      return hi;
+    }
+    return lo;
+  };
+  // Two component sets (300 rows) a CTA: enough rows to spread an iteration's
+  // exchange over (256 uneven beams, mixed: 2.36 ms at up to 300 rows, 3.06 at
+  // 150, 2.52 at 450), few enough to keep a slow model's iterations short;
+  // three only where a model needs them.
+  int sets = 2;
+  for (int m : order)
+    if ((eng.row_off[m + 1] - eng.row_off[m]) > (long long)grid_max * (sets * kSetRows * 8 / 9)) sets = kMaxSets;
+  plan(sets, team);
+  // queue order: the longest expected solve first, so that no long one starts
+  // last and the short ones fill the CTAs that the others free
+  std::vector<double> expect(M, 0.0);
+  int nloc_max = 0;
+  for (int m : order) {
+    const int n = eng.row_off[m + 1] - eng.row_off[m];
+    expect[m] = cost(Range{0, 0, expected_iterations(eng.models[m], eng.hosts[m])}, n, team[m]);
+    nloc_max = std::max(nloc_max, (n + team[m] - 1) / team[m]);
+  }
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return expect[x] > expect[y]; });
+  // component sets of the launch (the kernel's register steps go by them);
+  // parts of equal weight differ in their rows
+  sets = std::min(kMaxSets, (nloc_max + nloc_max / 8 + kSetRows - 1) / kSetRows);
+  std::vector<TeamSplit> split(M);
+  std::atomic<bool> good(true);
+  // few models: threads within each split, else one model per thread
+  const int threads = host_threads(), across = (int)order.size() >= threads ? threads : 1;
+  parallel_for((int)order.size(), across, [&](int, int i) {
+    const int m = order[i], a = eng.row_off[m], n = eng.row_off[m + 1] - a;
+    for (int k = team[m]; good; k = std::min({grid_max, n, k + std::max(1, k / 10)})) {
+      // the largest team streams what does not fit
+      const bool last = k >= std::min(grid_max, n);
+      if (team_split_model(a, n, k, sets, rowptr, col, eng.models[m].rest.data(), eng.hosts[m].act_node.data(), mt,
+                           dil, budget, last, across > 1 || n < 4096 ? 1 : threads, split[m]))
+        break;
+      if (last) good = false;
+    }
   });
+  if (!good) return false;
   out = TeamHost();
-  out.pub.assign(R, 0);
+  out.pub.resize(R);
   std::vector<unsigned char> rpub(R, 0);
   for (int m : order) {
-    const int a = eng.row_off[m], n = eng.row_off[m + 1] - a;
-    const long long nb = rowptr[a + n] - rowptr[a];
-    const size_t need = team_layout(n, (int)std::min<long long>(nb, 1 << 28), 0, mt, dil).total;
-    int k = std::max({1, n <= kAloneRows ? 1 : (n + want - 1) / want, (int)((need + budget - 1) / budget), (n + kTeamMaxRows - 1) / kTeamMaxRows});
-    TeamSplit sp;
-    for (;; k += std::max(1, k / 10)) {
-      if (k > std::min(grid_max, n)) return false;
-      if (team_split_model(a, n, k, rowptr, col, eng.models[m].rest.data(), eng.hosts[m].act_node.data(), mt, dil,
-                           budget, sp))
-        break;
-    }
+    TeamSplit& sp = split[m];
     const int s0 = (int)out.slots.size();
-    const int r0 = (int)out.rows.size(), ro0 = (int)out.ro.size(), h0 = (int)out.halo.size(), b0 = (int)out.cl.size();
-    for (TeamSlot s : sp.slots) {
+    std::copy(sp.pub.begin(), sp.pub.end(), rpub.begin() + eng.row_off[m]);
+    for (TeamSlot& s : sp.slots) {
       s.model = m;
       s.s0 = s0;
-      s.r0 += r0;
-      s.ro0 += ro0;
-      s.h0 += h0;
-      s.b0 += b0;
-      out.slots.push_back(s);
     }
-    for (int i = 0; i < n; i++) rpub[a + i] = sp.pub[i];
-    out.rows.insert(out.rows.end(), sp.rows.begin(), sp.rows.end());
-    out.ro.insert(out.ro.end(), sp.ro.begin(), sp.ro.end());
-    out.halo.insert(out.halo.end(), sp.halo.begin(), sp.halo.end());
-    out.cl.insert(out.cl.end(), sp.cl.begin(), sp.cl.end());
-    out.blk.insert(out.blk.end(), sp.blk.begin(), sp.blk.end());
-    out.nloc = std::max(out.nloc, sp.nloc_max);
-    out.smem = std::max(out.smem, sp.smem);
+    append_split(out, sp);
+    sp = TeamSplit();
   }
-  out.src.resize(out.rows.size());
-  out.dloc.resize(out.rows.size());
+  out.diag.resize(out.rows.size());
   for (size_t i = 0; i < out.rows.size(); i++) {
-    const int r = out.rows[i];
-    out.src[i] = rowptr[r];
-    // a row without blocks (an active node in no element) cannot be owned:
-    // its diagonal has no place in the slot
-    if (diag[r] < rowptr[r] || diag[r] >= rowptr[r + 1] || rowptr[r + 1] - rowptr[r] > 65535) return false;
-    out.dloc[i] = (unsigned short)(diag[r] - rowptr[r]);
-    out.pub[i] = rpub[r];
+    out.diag[i] = diag[out.rows[i]];
+    out.pub[i] = rpub[out.rows[i]];
   }
   out.grid = std::min(grid_max, (int)out.slots.size());
-  // lanes per row of the SpMV: as many as the row warps hold at once
-  out.lanes = out.nloc * 16 <= kRowThreads ? 16 : out.nloc * 8 <= kRowThreads ? 8 : 4;
-  out.sets = out.nloc > kSetRows ? 2 : 1;
+  out.sets = sets;
+  out.step_bytes = step_bytes(mt, dil);
   return true;
+}
+
+void team_parallel(int n, const std::function<void(int)>& f) {
+  parallel_for(n, host_threads(), [&](int, int i) { f(i); });
 }
 
 static std::mutex g_team_mu;
@@ -1215,9 +1547,10 @@ cudaError_t launch_pcg_team(Engine& eng, int max_iter, bool update_state, const 
   a.rows = d.team_rows;
   a.pub = d.team_pub;
   a.halo = d.team_halo;
-  a.ro = d.team_ro;
-  a.src = d.team_src;
-  a.dloc = d.team_dloc;
+  a.diag = d.team_diag;
+  a.group = d.team_group;
+  a.blk = d.team_blk;
+  a.stream = d.team_stream;
   a.cl = d.team_cl;
   a.g1 = d.team_g1;
   a.g2 = d.team_g2;
