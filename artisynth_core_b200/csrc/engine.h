@@ -11,6 +11,7 @@
 
 #include <cstdint>
 #include <functional>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -353,6 +354,8 @@ struct ElemGroup {
   int elem_inc = 0;  // ELEMENT soft incompressibility (one pressure per element)
 };
 
+struct HostStage;
+
 struct Engine {
   int device = 0;
   int precision = B200FEM_PREC_FP64;
@@ -438,6 +441,9 @@ struct Engine {
   float last_asm_ms = 0, last_solve_ms = 0, last_call_ms = 0;
   std::vector<double> last_step_params;
   b200fem_stats last_stats{};
+  // page-locked staging of large host arrays (api.cu: stage_copy), from the
+  // first such copy on
+  std::shared_ptr<HostStage> stage;
   std::vector<void*> allocations;
   size_t device_bytes = 0;  // sum of the allocations above
 };

@@ -30,6 +30,7 @@
 #include <cstdint>
 #include <mutex>
 #include <numeric>
+#include <system_error>
 #include <thread>
 #include <type_traits>
 
@@ -58,10 +59,6 @@ constexpr int kWantRows = 46, kWantTeam = 80, kAloneRows = 96;  // see plan_team
 constexpr double kExchangeRows = 165, kSetupRows = 3000, kFill = 0.95;  // see plan_team
 constexpr int kRowWeight = 8;  // a row's vectors, in blocks
 constexpr int kTeamMaxRestarts = 10;  // as in pcg.cu
-// The recurrences run on to this part of the tolerance (2-3 per cent more
-// iterations), so that the true residual that decides meets it in the first
-// round in spite of their drift.
-constexpr double kStopShort = 0.6;
 constexpr int kTeamRoundCap = 400;    // as in pcg.cu
 
 struct TeamArgs {
@@ -431,7 +428,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
         if (have_bb) return;
         collect();
         bb = sums[0];
-        thr2 = kStopShort * kStopShort * tol * tol * bb;
+        thr2 = tol * tol * bb;
         have_bb = true;
       };
       __syncthreads();  // C of P0
@@ -1097,7 +1094,10 @@ void parallel_for(int n, int threads, F&& f) {
     for (int i; (i = next++) < n;) f(th, i);
   };
   std::vector<std::thread> pool;
-  for (int th = 1; th < std::min(threads, n); th++) pool.emplace_back(work, th);
+  try {
+    for (int th = 1; th < std::min(threads, n); th++) pool.emplace_back(work, th);
+  } catch (const std::system_error&) {  // the system has no more threads: those there are do it
+  }
   work(0);
   for (auto& t : pool) t.join();
 }
@@ -1138,8 +1138,13 @@ void bisect(std::vector<int>& rows, int a, int b, int k, const double* pos, cons
     sum += weight[rows[mid++]];
   auto left = [&]() { bisect(rows, a, mid, kl, pos, node, weight, cut); };
   std::thread other;
-  if (b - a >= 8192) other = std::thread(left);
-  else left();
+  if (b - a >= 8192) {
+    try {
+      other = std::thread(left);
+    } catch (const std::system_error&) {
+    }
+  }
+  if (!other.joinable()) left();
   bisect(rows, mid, b, k - kl, pos, node, weight, cut + kl);
   if (other.joinable()) other.join();
 }
@@ -1477,7 +1482,7 @@ bool plan_team(Engine& eng, int grid_max, const std::vector<int>& rowptr, const 
       // the largest team streams what does not fit
       const bool last = k >= std::min(grid_max, n);
       if (team_split_model(a, n, k, sets, rowptr, col, eng.models[m].rest.data(), eng.hosts[m].act_node.data(), mt,
-                           dil, budget, last, across > 1 || n < 4096 ? 1 : threads, split[m]))
+                           dil, budget, last, across > 1 ? 1 : std::min(threads, 1 + n / 4096), split[m]))
         break;
       if (last) good = false;
     }

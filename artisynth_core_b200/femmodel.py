@@ -673,9 +673,22 @@ class FemPack:
 
     def setStates(self, xs=None, vs=None):
         e = self.engine()
-        xe = None if xs is None else np.ascontiguousarray(np.concatenate([np.asarray(x).reshape(-1, 3) for x in xs]).reshape(-1))
-        ve = None if vs is None else np.ascontiguousarray(np.concatenate([np.asarray(v).reshape(-1, 3) for v in vs]).reshape(-1))
-        e.call("b200fem_set_state", L.dptr(xe), L.dptr(ve))
+        e.call("b200fem_set_state", L.dptr(self._joined(0, xs)), L.dptr(self._joined(1, vs)))
+
+    def _joined(self, which, arrays):
+        """The models' arrays one after the other, in a buffer the pack keeps (a fresh one would take its page faults
+        on every call)."""
+        if arrays is None:
+            return None
+        arrays = [np.asarray(a).reshape(-1, 3) for a in arrays]
+        if any(a.dtype != np.float64 for a in arrays):
+            return np.ascontiguousarray(np.concatenate(arrays).reshape(-1))
+        n = sum(a.shape[0] for a in arrays)
+        bufs = self.__dict__.setdefault("_join_buf", [None, None])
+        if bufs[which] is None or bufs[which].shape[0] != n:
+            bufs[which] = np.empty((n, 3))
+        np.concatenate(arrays, out=bufs[which])
+        return bufs[which].reshape(-1)
 
     def getStates(self):
         e = self.engine()
