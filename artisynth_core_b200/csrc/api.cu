@@ -20,7 +20,6 @@
 
 namespace b200fem {
 
-cudaError_t launch_forces_only(Engine& eng);
 int pcg_max_grid(int device);
 int pcg_max_cta_pieces();
 size_t fused_elem_bytes(int elem_type, int mat_kind, bool fp32);
@@ -80,7 +79,7 @@ cudaError_t upload(Engine& eng, T** ptr, const std::vector<T>& v) {
 }  // namespace
 
 void free_pack(Engine& eng) {
-  for (cudaGraphExec_t* ex : {&eng.asm_exec, &eng.step_exec, &eng.host_exec})
+  for (cudaGraphExec_t* ex : {&eng.plain_exec, &eng.step_exec, &eng.host_exec})
     if (*ex) {
       cudaGraphExecDestroy(*ex);
       *ex = nullptr;
@@ -1850,11 +1849,10 @@ int b200fem_update_stress_stiffness(b200fem_handle h, const double* x, double* f
   if (x) CK(cudaMemcpyAsync(d.x, x, 3 * sizeof(double) * (size_t)d.n_nodes, cudaMemcpyHostToDevice, eng.stream));
   CK(launch_reset_status(eng));
   CK(cudaEventRecord(eng.ev[0], eng.stream));
-  CK(launch_assemble(eng, 1.0, 0.0, true));
+  CK(launch_assemble(eng, true));
   // the factored solve matrix of the last step reads divBlk and kp, which
   // this assembly has just replaced
   if (eng.factored) eng.have_matrix = false;
-  CK(launch_forces_only(eng));
   if (eng.att.active()) CK(launch_attach_reduce(eng));
   CK(cudaEventRecord(eng.ev[1], eng.stream));
   const size_t fbytes = 3 * sizeof(double) * (size_t)d.n_nodes, kbytes = 9 * sizeof(double) * (size_t)d.nnzb;
@@ -2019,29 +2017,38 @@ int backward_euler_steps(Engine& eng, const b200fem_step_params* p, int nsteps, 
     CK(cudaEventCreate(&e));
     eng.ev_pool.push_back(e);
   }
-  if (graphs && (eng.step_exec == nullptr || eng.step_exec_max_iter != max_iter)) {
-    // one captured graph per step: assembly (element kernels, block gather,
-    // RHS), an event record node between the phases (times each phase), and
-    // the solve (PCG); one launch per step leaves no gap between the phases
-    for (cudaGraphExec_t* ex : {&eng.asm_exec, &eng.step_exec, &eng.host_exec})
+  if (graphs && eng.step_exec_max_iter != max_iter) {
+    for (cudaGraphExec_t* ex : {&eng.plain_exec, &eng.step_exec, &eng.host_exec})
       if (*ex) {
         cudaGraphExecDestroy(*ex);
         *ex = nullptr;
       }
+    eng.step_exec_max_iter = max_iter;
+  }
+  // One captured graph per step: the assembly and the solve, so one launch
+  // per step leaves no gap between the phases.  The last step's also holds
+  // the event records that time the phases; the steps before it go without
+  // them (about 7 us a step of a small beam).
+  auto capture_step = [&](bool timed, cudaGraphExec_t* exec) -> int {
+    if (*exec) return B200FEM_OK;
     cudaGraph_t graph = nullptr;
+    const unsigned ext = cudaEventRecordExternal;  // (a plain record inside a capture only orders work)
     CK(cudaStreamBeginCapture(eng.stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t ce = launch_assemble(eng, 0, 0, false);
-    if (ce == cudaSuccess) ce = launch_rhs(eng);
-    // (an external record node: a plain record inside a capture only orders work)
-    if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(eng.ev_pool[1], eng.stream, cudaEventRecordExternal);
+    cudaError_t ce = launch_assemble(eng, false);
+    if (ce == cudaSuccess && timed) ce = cudaEventRecordWithFlags(eng.ev_pool[1], eng.stream, ext);
     if (ce == cudaSuccess) ce = launch_solve(eng, max_iter);
     cudaError_t ee = cudaStreamEndCapture(eng.stream, &graph);
     if (ce != cudaSuccess) return cuda_fail(&eng, ce, "capture of the BackwardEuler step");
     if (ee != cudaSuccess) return cuda_fail(&eng, ee, "cudaStreamEndCapture");
-    ce = cudaGraphInstantiate(&eng.step_exec, graph, 0);
+    ce = cudaGraphInstantiate(exec, graph, 0);
     cudaGraphDestroy(graph);
     if (ce != cudaSuccess) return cuda_fail(&eng, ce, "cudaGraphInstantiate");
-    eng.step_exec_max_iter = max_iter;
+    return B200FEM_OK;
+  };
+  if (graphs && !host_graph) {
+    int st = capture_step(true, &eng.step_exec);
+    if (st == B200FEM_OK && nsteps > 1) st = capture_step(false, &eng.plain_exec);
+    if (st != B200FEM_OK) return st;
   }
   const size_t state_bytes = 3 * sizeof(double) * (size_t)d.n_nodes;
   if (host_graph) {
@@ -2060,9 +2067,8 @@ int backward_euler_steps(Engine& eng, const b200fem_step_params* p, int nsteps, 
       if (ce == cudaSuccess) ce = launch_reset_status(eng);
       if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(eng.ev[0], eng.stream, ext);
       if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(eng.ev_pool[0], eng.stream, ext);
-      if (ce == cudaSuccess) ce = launch_assemble(eng, 0, 0, false);
-      if (ce == cudaSuccess) ce = launch_rhs(eng);
-      if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(eng.ev_pool[1], eng.stream, ext);
+      if (ce == cudaSuccess) ce = launch_assemble(eng, false);
+        if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(eng.ev_pool[1], eng.stream, ext);
       if (ce == cudaSuccess) ce = launch_solve(eng, max_iter);
       if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(eng.ev_pool[2], eng.stream, ext);
       if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(eng.ev[1], eng.stream, ext);
@@ -2094,12 +2100,12 @@ int backward_euler_steps(Engine& eng, const b200fem_step_params* p, int nsteps, 
   if (v_host) CK(cudaMemcpyAsync(d.v, v_host, state_bytes, cudaMemcpyHostToDevice, eng.stream));
   CK(cudaEventRecord(eng.ev[0], eng.stream));
   for (int s = 0; s < nsteps; s++) {
-    CK(cudaEventRecord(eng.ev_pool[0], eng.stream));
+    const bool last = s == nsteps - 1;
+    if (last) CK(cudaEventRecord(eng.ev_pool[0], eng.stream));
     if (graphs) {
-      CK(cudaGraphLaunch(eng.step_exec, eng.stream));
+      CK(cudaGraphLaunch(last ? eng.step_exec : eng.plain_exec, eng.stream));
     } else {
-      CK(launch_assemble(eng, 0, 0, false));
-      CK(launch_rhs(eng));
+      CK(launch_assemble(eng, false));
       CK(cudaEventRecord(eng.ev_pool[1], eng.stream));
       if (p->abort_on_inverted) {
         int flags[4];
@@ -2110,7 +2116,7 @@ int backward_euler_steps(Engine& eng, const b200fem_step_params* p, int nsteps, 
       }
       CK(launch_solve(eng, max_iter));
     }
-    CK(cudaEventRecord(eng.ev_pool[2], eng.stream));
+    if (last) CK(cudaEventRecord(eng.ev_pool[2], eng.stream));
   }
   CK(cudaEventRecord(eng.ev[1], eng.stream));
   if (x_host) CK(cudaMemcpyAsync(x_host, d.x, state_bytes, cudaMemcpyDeviceToHost, eng.stream));

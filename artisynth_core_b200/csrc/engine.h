@@ -429,8 +429,8 @@ struct Engine {
   int pcg_variant = 0;
   int pcg_row_lanes = 16;  // lanes per block row in the PCG SpMV (tunable)
   // captured BackwardEuler step (element, gather, RHS, PCG) and its events
-  cudaGraphExec_t asm_exec = nullptr;
-  cudaGraphExec_t step_exec = nullptr;
+  cudaGraphExec_t step_exec = nullptr;   // with the events (the last step of a call)
+  cudaGraphExec_t plain_exec = nullptr;  // without
   int step_exec_max_iter = -1;
   // one step from page-locked host state as one graph (the buffers it holds)
   cudaGraphExec_t host_exec = nullptr;
@@ -506,8 +506,7 @@ cudaError_t launch_pcg_team(Engine& eng, int max_iter, bool update_state, const 
                             double tol_override, double* model_out);
 
 // kernels.cu
-cudaError_t launch_assemble(Engine& eng, double cK, double cM, bool want_K);
-cudaError_t launch_rhs(Engine& eng);
+cudaError_t launch_assemble(Engine& eng, bool want_K);
 cudaError_t launch_reset_status(Engine& eng);
 cudaError_t launch_pcg(Engine& eng, int max_iter, bool update_state, int init_zero);
 cudaError_t launch_pcg_on(Engine& eng, int max_iter, bool update_state, const double* rhs, double* xsol,

@@ -711,6 +711,107 @@ __global__ void __launch_bounds__(256) elem_linear_kernel(ElemArgs a, int corota
 }
 
 // ---------------------------------------------------------------------------
+// nodal forces and BackwardEuler right-hand side
+//   f_int(n) = sum of element stress forces at n
+//   b = M v0 + h (m g + f_ext - f_int)
+// (the mass- and stiffness-damping terms of updateNodeForces and the
+// b += (h alpha M + h beta K) v0 term of backwardEuler cancel exactly,
+// MechSystemSolver.java:2194-2301, FemModel3d.java:2783-2843)
+// ---------------------------------------------------------------------------
+struct RowsArgs {
+  int N;
+  const int *inc_ptr, *inc_idx;
+  const double* elemF;
+  const int *sidx, *node_model;
+  const double *mass, *v, *fext, *step;
+  double* fint;
+  double *b, *sol0;  // null: the nodal forces only
+  const int* active;
+  const double *vprev, *vprev2, *vprev3, *vprev4;
+  const double* row_nrm;
+};
+__device__ __forceinline__ void rows_node(const RowsArgs& ra, int n) {
+  if (n >= ra.N) return;
+  const int *__restrict__ inc_ptr = ra.inc_ptr, *__restrict__ inc_idx = ra.inc_idx, *__restrict__ sidx = ra.sidx,
+            *__restrict__ node_model = ra.node_model, *__restrict__ active = ra.active;
+  const double *__restrict__ elemF = ra.elemF, *__restrict__ mass = ra.mass, *__restrict__ v = ra.v,
+               *__restrict__ fext = ra.fext, *__restrict__ step = ra.step, *__restrict__ vprev = ra.vprev,
+               *__restrict__ vprev2 = ra.vprev2, *__restrict__ vprev3 = ra.vprev3, *__restrict__ vprev4 = ra.vprev4,
+               *__restrict__ row_nrm = ra.row_nrm;
+  double *__restrict__ fint = ra.fint, *__restrict__ b = ra.b, *__restrict__ sol0 = ra.sol0;
+  if (active && !active[node_model[n]]) return;  // model left out of this step
+  double f[3] = {0, 0, 0};
+  const int i0 = inc_ptr[n], i1 = inc_ptr[n + 1];
+  // four incidences per round: their index and force loads are independent
+  for (int i = i0; i < i1; i += 4) {
+    int idx[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) idx[k] = (i + k < i1) ? inc_idx[i + k] : -1;
+    double g[4][3];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+#pragma unroll
+      for (int c = 0; c < 3; c++) g[k][c] = idx[k] >= 0 ? (double)elemF[(size_t)idx[k] * 3 + c] : 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+#pragma unroll
+      for (int c = 0; c < 3; c++) f[c] += g[k][c];
+  }
+  if (fint) {
+    fint[3 * (size_t)n] = f[0];
+    fint[3 * (size_t)n + 1] = f[1];
+    fint[3 * (size_t)n + 2] = f[2];
+  }
+  int r = sidx[n];
+  if (b && r >= 0) {
+    const double* sp = step + (size_t)node_model[n] * 8;
+    double h = sp[0], m = mass[n];
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+      b[3 * (size_t)r + c] = m * v[3 * (size_t)n + c] + h * (m * sp[3 + c] + fext[3 * (size_t)n + c] - f[c]);
+    // the PCG starts from the current velocity, or from its extrapolation
+    // v + (v - v_prev) over the last two steps
+    if (sol0) {
+      double s0[3];
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const double vc = v[3 * (size_t)n + c];
+        if (vprev4)  // quartic through the last five velocities
+          s0[c] = 5.0 * (vc - vprev3[3 * (size_t)n + c]) + 10.0 * (vprev2[3 * (size_t)n + c] - vprev[3 * (size_t)n + c]) +
+                  vprev4[3 * (size_t)n + c];
+        else if (vprev3)  // cubic through the last four velocities
+          s0[c] = 4.0 * (vc + vprev2[3 * (size_t)n + c]) - 6.0 * vprev[3 * (size_t)n + c] - vprev3[3 * (size_t)n + c];
+        else if (vprev2)  // quadratic through the last three velocities
+          s0[c] = 3.0 * (vc - vprev[3 * (size_t)n + c]) + vprev2[3 * (size_t)n + c];
+        else
+          s0[c] = vprev ? 2.0 * vc - vprev[3 * (size_t)n + c] : vc;
+      }
+      if (row_nrm) {
+        // plane constraint: the initial guess lies on the plane
+        const double* q = row_nrm + 3 * (size_t)r;
+        const double d = q[0] * s0[0] + q[1] * s0[1] + q[2] * s0[2];
+#pragma unroll
+        for (int c = 0; c < 3; c++) s0[c] -= q[c] * d;
+      }
+#pragma unroll
+      for (int c = 0; c < 3; c++) sol0[3 * (size_t)r + c] = s0[c];
+    }
+  }
+}
+__global__ void rows_kernel(RowsArgs ra) { rows_node(ra, blockIdx.x * blockDim.x + threadIdx.x); }
+
+// The gathers below also run the nodal rows, in the first blocks of their
+// grid: both read what the element kernel wrote and neither reads the other,
+// and one launch in place of two leaves out a launch gap and the rows' own
+// time (40x10x10 hex beam: 38 -> 34.5 us of assembly; 72-row beam 26 -> 18.4).
+constexpr int kGatherThreads = 256;
+__device__ __forceinline__ bool gather_rows_part(const RowsArgs& ra, int rows_blocks) {
+  if ((int)blockIdx.x >= rows_blocks) return false;
+  rows_node(ra, blockIdx.x * kGatherThreads + threadIdx.x);
+  return true;
+}
+
+// ---------------------------------------------------------------------------
 // block gather: one thread per upper block (diagonal included), taken from
 // the list of the pattern's upper blocks, so every lane of a warp sums a
 // block.  The sums: the contribution list in element order, then the NODAL
@@ -720,15 +821,16 @@ __global__ void __launch_bounds__(256) elem_linear_kernel(ElemArgs a, int corota
 // (FemModel3d.java:3003-3026) and lower blocks are never summed.
 // ---------------------------------------------------------------------------
 template <typename TK, typename TO>
-__global__ void __launch_bounds__(256) gather_block_kernel(
+__global__ void __launch_bounds__(kGatherThreads) gather_block_kernel(
     long long n_up, const int* __restrict__ up, const int* __restrict__ cptr, const int* __restrict__ cidx,
     const TK* __restrict__ elemK, const int* __restrict__ blk_row, const int* __restrict__ blk_diag,
     const int* __restrict__ row_model, const int* __restrict__ act_node, const double* __restrict__ mass,
     const double* __restrict__ step, int mode, TO* __restrict__ out, const int* __restrict__ dptr,
     const int* __restrict__ didx, const double* __restrict__ divblk, const double* __restrict__ node_kp,
     const int* __restrict__ active, const int* __restrict__ mirror, const int* __restrict__ dst,
-    const int* __restrict__ mdst) {
-  const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int* __restrict__ mdst, RowsArgs ra, int rows_blocks) {
+  if (gather_rows_part(ra, rows_blocks)) return;
+  const long long q = (long long)(blockIdx.x - rows_blocks) * kGatherThreads + threadIdx.x;
   if (q >= n_up) return;
   const int p = up[q];
   const int row = blk_row[p];
@@ -815,16 +917,17 @@ __global__ void __launch_bounds__(256) gather_block_kernel(
 // not summed.
 // ---------------------------------------------------------------------------
 template <typename TK, typename TO>
-__global__ void __launch_bounds__(256) gather_staged_kernel(
+__global__ void __launch_bounds__(kGatherThreads) gather_staged_kernel(
     long long nnzb, const int* __restrict__ cptr, const int* __restrict__ cidx, const TK* __restrict__ elemK,
     const int* __restrict__ blk_row, const int* __restrict__ blk_diag, const int* __restrict__ row_model,
     const int* __restrict__ act_node, const double* __restrict__ mass, const double* __restrict__ step, int mode,
     TO* __restrict__ out, const int* __restrict__ dptr, const int* __restrict__ didx,
     const double* __restrict__ divblk, const double* __restrict__ node_kp, const int* __restrict__ active,
-    const int* __restrict__ mirror) {
+    const int* __restrict__ mirror, RowsArgs ra, int rows_blocks) {
   __shared__ TO stage[8][32 * 9];
+  if (gather_rows_part(ra, rows_blocks)) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long wbase = ((long long)blockIdx.x * 8 + warp) * 32;
+  const long long wbase = ((long long)(blockIdx.x - rows_blocks) * 8 + warp) * 32;
   const long long p = wbase + lane;
   TO* my = stage[warp] + lane * 9;
   bool live = p < nnzb;
@@ -915,86 +1018,6 @@ __global__ void __launch_bounds__(256) gather_staged_kernel(
     const int mq = mirror[q];
     if (mq >= 0 && mq < q) continue;  // lower block: written by its mirror
     o[i] = stage[warp][i];
-  }
-}
-
-// ---------------------------------------------------------------------------
-// nodal forces and BackwardEuler right-hand side
-//   f_int(n) = sum of element stress forces at n
-//   b = M v0 + h (m g + f_ext - f_int)
-// (the mass- and stiffness-damping terms of updateNodeForces and the
-// b += (h alpha M + h beta K) v0 term of backwardEuler cancel exactly,
-// MechSystemSolver.java:2194-2301, FemModel3d.java:2783-2843)
-// ---------------------------------------------------------------------------
-template <typename TF>
-__global__ void rows_kernel(int N, const int* __restrict__ inc_ptr, const int* __restrict__ inc_idx,
-                            const TF* __restrict__ elemF, const int* __restrict__ sidx,
-                            const int* __restrict__ node_model, const double* __restrict__ mass,
-                            const double* __restrict__ v, const double* __restrict__ fext,
-                            const double* __restrict__ step, double* __restrict__ fint,
-                            double* __restrict__ b, double* __restrict__ sol0, const int* __restrict__ active,
-                            const double* __restrict__ vprev, const double* __restrict__ vprev2,
-                            const double* __restrict__ vprev3, const double* __restrict__ vprev4,
-                            const double* __restrict__ row_nrm) {
-  int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  if (active && !active[node_model[n]]) return;  // model left out of this step
-  double f[3] = {0, 0, 0};
-  const int i0 = inc_ptr[n], i1 = inc_ptr[n + 1];
-  // four incidences per round: their index and force loads are independent
-  for (int i = i0; i < i1; i += 4) {
-    int idx[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) idx[k] = (i + k < i1) ? inc_idx[i + k] : -1;
-    double g[4][3];
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-#pragma unroll
-      for (int c = 0; c < 3; c++) g[k][c] = idx[k] >= 0 ? (double)elemF[(size_t)idx[k] * 3 + c] : 0.0;
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-#pragma unroll
-      for (int c = 0; c < 3; c++) f[c] += g[k][c];
-  }
-  if (fint) {
-    fint[3 * (size_t)n] = f[0];
-    fint[3 * (size_t)n + 1] = f[1];
-    fint[3 * (size_t)n + 2] = f[2];
-  }
-  int r = sidx[n];
-  if (b && r >= 0) {
-    const double* sp = step + (size_t)node_model[n] * 8;
-    double h = sp[0], m = mass[n];
-#pragma unroll
-    for (int c = 0; c < 3; c++)
-      b[3 * (size_t)r + c] = m * v[3 * (size_t)n + c] + h * (m * sp[3 + c] + fext[3 * (size_t)n + c] - f[c]);
-    // the PCG starts from the current velocity, or from its extrapolation
-    // v + (v - v_prev) over the last two steps
-    if (sol0) {
-      double s0[3];
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const double vc = v[3 * (size_t)n + c];
-        if (vprev4)  // quartic through the last five velocities
-          s0[c] = 5.0 * (vc - vprev3[3 * (size_t)n + c]) + 10.0 * (vprev2[3 * (size_t)n + c] - vprev[3 * (size_t)n + c]) +
-                  vprev4[3 * (size_t)n + c];
-        else if (vprev3)  // cubic through the last four velocities
-          s0[c] = 4.0 * (vc + vprev2[3 * (size_t)n + c]) - 6.0 * vprev[3 * (size_t)n + c] - vprev3[3 * (size_t)n + c];
-        else if (vprev2)  // quadratic through the last three velocities
-          s0[c] = 3.0 * (vc - vprev[3 * (size_t)n + c]) + vprev2[3 * (size_t)n + c];
-        else
-          s0[c] = vprev ? 2.0 * vc - vprev[3 * (size_t)n + c] : vc;
-      }
-      if (row_nrm) {
-        // plane constraint: the initial guess lies on the plane
-        const double* q = row_nrm + 3 * (size_t)r;
-        const double d = q[0] * s0[0] + q[1] * s0[1] + q[2] * s0[2];
-#pragma unroll
-        for (int c = 0; c < 3; c++) s0[c] -= q[c] * d;
-      }
-#pragma unroll
-      for (int c = 0; c < 3; c++) sol0[3 * (size_t)r + c] = s0[c];
-    }
   }
 }
 
@@ -2386,18 +2409,56 @@ static cudaError_t launch_assemble_fused(Engine& eng) {
   return launch_fused_blocks(eng, eng.fused_chunks);
 }
 
-cudaError_t launch_assemble(Engine& eng, double cK, double cM, bool want_K) {
-  (void)cK;
-  (void)cM;
+static RowsArgs rows_args(Engine& eng, double* b, double* sol) {
+  DevPack& d = eng.d;
+  RowsArgs ra{};
+  ra.N = d.n_nodes;
+  ra.inc_ptr = d.inc_ptr;
+  ra.inc_idx = d.inc_idx;
+  ra.elemF = d.elemF;  // nodal forces are FP64 in both forms
+  ra.sidx = d.sidx;
+  ra.node_model = d.node_model;
+  ra.mass = d.mass;
+  ra.v = d.v;
+  ra.fext = d.fext;
+  ra.step = d.step;
+  ra.fint = d.fint;
+  ra.b = b;
+  ra.sol0 = sol;
+  ra.active = eng.any_inactive ? d.model_active : nullptr;
+  ra.vprev = eng.opt_warm_start >= 1 ? d.vprev : nullptr;
+  ra.vprev2 = eng.opt_warm_start >= 2 ? d.vprev2 : nullptr;
+  ra.vprev3 = eng.opt_warm_start >= 3 ? d.vprev3 : nullptr;
+  ra.vprev4 = eng.opt_warm_start == 4 ? d.vprev4 : nullptr;
+  ra.row_nrm =
+      (sol && eng.integrator == B200FEM_INTEGRATOR_CONSTRAINED_BACKWARD_EULER && d.row_nrm) ? d.row_nrm : nullptr;
+  return ra;
+}
+
+static cudaError_t launch_rows(Engine& eng, double* b, double* sol) {
+  const int threads = 64, blocks = (eng.d.n_nodes + threads - 1) / threads;
+  rows_kernel<<<blocks, threads, 0, eng.stream>>>(rows_args(eng, b, sol));
+  return cudaGetLastError();
+}
+
+// The element kernels, then the matrix (K for want_K, else the step's solve
+// matrix) with the nodal rows.
+cudaError_t launch_assemble(Engine& eng, bool want_K) {
   cudaError_t e = cudaSuccess;
   DevPack& d = eng.d;
   const bool fp32 = eng.precision == B200FEM_PREC_MIXED;
-  if (!want_K && eng.fused) return launch_assemble_fused(eng);
+  // K: the nodal forces; the step: also the right-hand side and the PCG's
+  // initial guess
+  double *const b = want_K ? nullptr : d.b, *const sol = want_K ? nullptr : d.sol;
+  if (!want_K && eng.fused) {
+    if ((e = launch_assemble_fused(eng)) != cudaSuccess) return e;
+    return launch_rows(eng, b, sol);
+  }
   if ((e = launch_nodal_pressure(eng)) != cudaSuccess) return e;
   if ((e = launch_divblk(eng)) != cudaSuccess) return e;
   if ((e = launch_element_pressure(eng)) != cudaSuccess) return e;
   // the step on the node-row path: S, the nodal forces, b and the PCG's
-  // initial guess in one launch per group (launch_rhs then has nothing left)
+  // initial guess in one launch per group
   if (!want_K && eng.tet_rows) return launch_tet_rows(eng, false);
   for (const ElemGroup& g : eng.groups) {
     e = by_elem_type(g.elem_type, [&](auto tag) {
@@ -2407,20 +2468,22 @@ cudaError_t launch_assemble(Engine& eng, double cK, double cM, bool want_K) {
     if (e != cudaSuccess) return e;
   }
   const int* act = eng.any_inactive ? d.model_active : nullptr;
-  if (d.n_up == 0) return cudaSuccess;
+  if (d.n_up == 0) return launch_rows(eng, b, sol);
+  const RowsArgs ra = rows_args(eng, b, sol);
+  const int rb = (d.n_nodes + kGatherThreads - 1) / kGatherThreads;
   if (!want_K && eng.factored) {
     // the step's factored solve matrix: the direct blocks into S1, without
     // the dilational triples (the PCG applies that term from divBlk)
-    if (d.n_up1 == 0) return cudaSuccess;
+    if (d.n_up1 == 0) return launch_rows(eng, b, sol);
     const unsigned blocks = (unsigned)((d.n_up1 + 255) / 256);
     if (fp32)
-      gather_block_kernel<float, float><<<blocks, 256, 0, eng.stream>>>(
+      gather_block_kernel<float, float><<<blocks + rb, kGatherThreads, 0, eng.stream>>>(
           d.n_up1, d.up1, d.contrib_ptr, d.contrib_idx, d.elemK_f, d.blk_row, d.blk_diag, d.row_model, d.act_node,
-          d.mass, d.step, 1, d.S1_f, nullptr, nullptr, nullptr, nullptr, act, d.blk_mirror, d.up1_dst, d.up1_mdst);
+          d.mass, d.step, 1, d.S1_f, nullptr, nullptr, nullptr, nullptr, act, d.blk_mirror, d.up1_dst, d.up1_mdst, ra, rb);
     else
-      gather_block_kernel<double, double><<<blocks, 256, 0, eng.stream>>>(
+      gather_block_kernel<double, double><<<blocks + rb, kGatherThreads, 0, eng.stream>>>(
           d.n_up1, d.up1, d.contrib_ptr, d.contrib_idx, d.elemK, d.blk_row, d.blk_diag, d.row_model, d.act_node,
-          d.mass, d.step, 1, d.S1, nullptr, nullptr, nullptr, nullptr, act, d.blk_mirror, d.up1_dst, d.up1_mdst);
+          d.mass, d.step, 1, d.S1, nullptr, nullptr, nullptr, nullptr, act, d.blk_mirror, d.up1_dst, d.up1_mdst, ra, rb);
     return cudaGetLastError();
   }
   // Matrices that stay in L2 (up to 64 MB of blocks): one thread per block
@@ -2433,17 +2496,17 @@ cudaError_t launch_assemble(Engine& eng, double cK, double cM, bool want_K) {
     const unsigned sb = (unsigned)((d.nnzb + 255) / 256);
     if (fp32) {
       if (want_K)
-        gather_staged_kernel<float, double><<<sb, 256, 0, eng.stream>>>(
+        gather_staged_kernel<float, double><<<sb + rb, kGatherThreads, 0, eng.stream>>>(
             d.nnzb, d.contrib_ptr, d.contrib_idx, d.elemK_f, d.blk_row, d.blk_diag, d.row_model, d.act_node, d.mass,
-            d.step, 0, d.K, d.dil_ptr, d.dil_idx, d.divblk, d.node_kp, act, d.blk_mirror);
+            d.step, 0, d.K, d.dil_ptr, d.dil_idx, d.divblk, d.node_kp, act, d.blk_mirror, ra, rb);
       else
-        gather_staged_kernel<float, float><<<sb, 256, 0, eng.stream>>>(
+        gather_staged_kernel<float, float><<<sb + rb, kGatherThreads, 0, eng.stream>>>(
             d.nnzb, d.contrib_ptr, d.contrib_idx, d.elemK_f, d.blk_row, d.blk_diag, d.row_model, d.act_node, d.mass,
-            d.step, 1, d.S_f, d.dil_ptr, d.dil_idx, d.divblk, d.node_kp, act, d.blk_mirror);
+            d.step, 1, d.S_f, d.dil_ptr, d.dil_idx, d.divblk, d.node_kp, act, d.blk_mirror, ra, rb);
     } else {
-      gather_staged_kernel<double, double><<<sb, 256, 0, eng.stream>>>(
+      gather_staged_kernel<double, double><<<sb + rb, kGatherThreads, 0, eng.stream>>>(
           d.nnzb, d.contrib_ptr, d.contrib_idx, d.elemK, d.blk_row, d.blk_diag, d.row_model, d.act_node, d.mass,
-          d.step, want_K ? 0 : 1, want_K ? d.K : d.S, d.dil_ptr, d.dil_idx, d.divblk, d.node_kp, act, d.blk_mirror);
+          d.step, want_K ? 0 : 1, want_K ? d.K : d.S, d.dil_ptr, d.dil_idx, d.divblk, d.node_kp, act, d.blk_mirror, ra, rb);
     }
     return cudaGetLastError();
   }
@@ -2451,18 +2514,18 @@ cudaError_t launch_assemble(Engine& eng, double cK, double cM, bool want_K) {
   const unsigned blocks = (unsigned)((d.n_up + 255) / 256);
   if (fp32) {
     if (want_K)
-      gather_block_kernel<float, double><<<blocks, 256, 0, eng.stream>>>(
+      gather_block_kernel<float, double><<<blocks + rb, kGatherThreads, 0, eng.stream>>>(
           d.n_up, d.up_blocks, d.contrib_ptr, d.contrib_idx, d.elemK_f, d.blk_row, d.blk_diag, d.row_model,
-          d.act_node, d.mass, d.step, 0, d.K, d.dil_ptr, d.dil_idx, d.divblk, d.node_kp, act, d.blk_mirror, nullptr, nullptr);
+          d.act_node, d.mass, d.step, 0, d.K, d.dil_ptr, d.dil_idx, d.divblk, d.node_kp, act, d.blk_mirror, nullptr, nullptr, ra, rb);
     else
-      gather_block_kernel<float, float><<<blocks, 256, 0, eng.stream>>>(
+      gather_block_kernel<float, float><<<blocks + rb, kGatherThreads, 0, eng.stream>>>(
           d.n_up, d.up_blocks, d.contrib_ptr, d.contrib_idx, d.elemK_f, d.blk_row, d.blk_diag, d.row_model,
-          d.act_node, d.mass, d.step, 1, d.S_f, d.dil_ptr, d.dil_idx, d.divblk, d.node_kp, act, d.blk_mirror, nullptr, nullptr);
+          d.act_node, d.mass, d.step, 1, d.S_f, d.dil_ptr, d.dil_idx, d.divblk, d.node_kp, act, d.blk_mirror, nullptr, nullptr, ra, rb);
   } else {
-    gather_block_kernel<double, double><<<blocks, 256, 0, eng.stream>>>(
+    gather_block_kernel<double, double><<<blocks + rb, kGatherThreads, 0, eng.stream>>>(
         d.n_up, d.up_blocks, d.contrib_ptr, d.contrib_idx, d.elemK, d.blk_row, d.blk_diag, d.row_model,
         d.act_node, d.mass, d.step, want_K ? 0 : 1, want_K ? d.K : d.S, d.dil_ptr, d.dil_idx, d.divblk,
-        d.node_kp, act, d.blk_mirror, nullptr, nullptr);
+        d.node_kp, act, d.blk_mirror, nullptr, nullptr, ra, rb);
   }
   return cudaGetLastError();
 }
@@ -2494,30 +2557,6 @@ cudaError_t launch_reset_status(Engine& eng) {
   reset_status_kernel<<<1, 32, 0, eng.stream>>>(eng.d.flags, (long long*)eng.d.dmin);
   return cudaGetLastError();
 }
-
-static cudaError_t launch_rows(Engine& eng, double* b, double* sol) {
-  DevPack& d = eng.d;
-  const int threads = 64;
-  const int blocks = (d.n_nodes + threads - 1) / threads;
-  const int* act = eng.any_inactive ? d.model_active : nullptr;
-  const double* vp = eng.opt_warm_start >= 1 ? d.vprev : nullptr;
-  const double* vp2 = eng.opt_warm_start >= 2 ? d.vprev2 : nullptr;
-  const double* vp3 = eng.opt_warm_start >= 3 ? d.vprev3 : nullptr;
-  const double* vp4 = eng.opt_warm_start == 4 ? d.vprev4 : nullptr;
-  const double* nrm =
-      (sol && eng.integrator == B200FEM_INTEGRATOR_CONSTRAINED_BACKWARD_EULER && d.row_nrm) ? d.row_nrm : nullptr;
-  // nodal forces are FP64 in both forms
-  rows_kernel<double><<<blocks, threads, 0, eng.stream>>>(d.n_nodes, d.inc_ptr, d.inc_idx, d.elemF, d.sidx,
-                                                         d.node_model, d.mass, d.v, d.fext, d.step, d.fint, b, sol, act, vp,
-                                                         vp2, vp3, vp4, nrm);
-  return cudaGetLastError();
-}
-
-// follows launch_assemble(..., want_K = false) in the step; the node-row
-// path has formed b and the initial guess already
-cudaError_t launch_rhs(Engine& eng) { return eng.tet_rows ? cudaSuccess : launch_rows(eng, eng.d.b, eng.d.sol); }
-
-cudaError_t launch_forces_only(Engine& eng) { return launch_rows(eng, nullptr, nullptr); }
 
 cudaError_t launch_spmv(Engine& eng, const double* x, double* y) {
   DevPack& d = eng.d;
