@@ -1176,14 +1176,18 @@ bool all_finite_arrays(std::initializer_list<std::pair<const double*, size_t>> a
 // Small or page-locked arrays take plain asynchronous copies on the engine's
 // stream.  Staged copies are complete on return; either way the caller
 // synchronises the stream before it reads.
+// (kStageMin: an update's 16 MB take 2.2 ms staged and 3.6 plain, 4 MB 1.4 and
+// 1.2: below it the threads cost more than they save)
+constexpr size_t kStageMin = 6 << 20;
 cudaError_t stage_copy(Engine& eng, std::initializer_list<HostCopy> list, bool to_host) {
   const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
   std::vector<HostCopy> chunks;
   cudaError_t e = cudaSuccess;
-  size_t staged = 0;
+  size_t staged = 0, total = 0;
+  for (const HostCopy& c : list) total += c.host ? c.bytes : 0;
   for (const HostCopy& c : list) {
     if (!c.host || c.bytes == 0) continue;
-    bool pageable = c.bytes >= HostStage::kChunk;
+    bool pageable = total >= kStageMin && c.bytes >= HostStage::kChunk;
     if (pageable) {
       cudaPointerAttributes at{};
       if (cudaPointerGetAttributes(&at, c.host) != cudaSuccess) cudaGetLastError();

@@ -1,5 +1,5 @@
-"""Host arrays of every size come back as they went in: below and above the 1 MiB from which pageable arrays are
-staged in chunks, a last chunk of a few values, page-locked arrays; a non-finite value anywhere is refused before
+"""Host arrays of every size come back as they went in: below and above the 6 MiB of x and v together from which
+pageable arrays are staged in chunks of 1 MiB, a last chunk of a few values, page-locked arrays; a non-finite value anywhere is refused before
 the device's state changes; the stiffness arrays of an update equal the ones of the device's other exports."""
 import numpy as np
 import pytest
@@ -24,7 +24,7 @@ def _model(n_nodes):
     return wl.model()
 
 
-@pytest.mark.parametrize("n", [5, 43690, 43691, 87383, 131075])
+@pytest.mark.parametrize("n", [5, 43691, 131072, 131073, 174763])
 def test_state_round_trip(n, b200):
     m = _model(n)
     rng = np.random.default_rng(n)
@@ -45,7 +45,7 @@ def test_state_round_trip(n, b200):
 def test_page_locked_arrays(b200):
     import torch
 
-    n = 90000
+    n = 140000
     m = _model(n)
     x = torch.randn(3 * n, dtype=torch.float64).pin_memory().numpy()
     v = torch.randn(3 * n, dtype=torch.float64).pin_memory().numpy()
