@@ -324,11 +324,12 @@ int b200fem_memory_usage(b200fem_handle h, unsigned long long* bytes);
                                     resident when they fit); 2 strided: every model cut
                                     into short pieces dealt over all CTAs; 3 cluster: one
                                     thread-block cluster per model, models taken from a
-                                    queue largest first.  Auto: contiguous when the rows fit
-                                    shared-memory residency or the handle has one model,
-                                    else strided (on the 256-beam pack the strided split
-                                    measured 10.1 ms per step against the cluster split's
-                                    14.2: the slowest model is held to one cluster) */
+                                    queue largest first.  Auto: one team of CTAs per model
+                                    (pcg_team.cu) wherever every model fits one; the split
+                                    reported, and used where one does not, is contiguous
+                                    when the rows fit shared-memory residency or the handle
+                                    has one model, else strided (the 256-beam pack, solve
+                                    per step: teams 2.4 ms, strided 11.5, cluster 14.2) */
 #define B200FEM_OPT_ROW_LANES 2  /* lanes per block row in the iteration SpMV: 0 auto, 4, 8, 16, 32 */
 #define B200FEM_OPT_PCG_CTAS 3   /* CTAs of the persistent PCG kernel: 0 auto (one per SM) */
 #define B200FEM_OPT_PIECE_ROWS 4 /* block rows per piece in the strided split: 0 auto (64) */
