@@ -9,19 +9,24 @@
 //   * the CTA's blocks of S stay in registers and shared memory for the whole
 //     solve (what exceeds them is streamed from a copy in the order the lanes
 //     read it) and the PCG vectors in the registers of the lanes that own them;
-//   * there is no barrier: every value that crosses CTAs travels as a 16-byte
-//     packet {double, tag} written and read in one 128-bit access, so the
-//     reader polls the datum itself and one L2 round trip carries both the
+//   * there is no grid barrier: every value that crosses CTAs travels in a
+//     16-byte packet with a tag, written and read in one 128-bit access, so
+//     the reader polls the datum itself and one L2 round trip carries both the
 //     value and the synchronisation.  A reader waits for the rows next to its
 //     own and for the team's k partial sums, nothing else;
 //   * models run independently of one another: teams form from a queue of
-//     slots (largest models first), so a slow model occupies its own CTAs
-//     instead of keeping the grid in its loop.
+//     slots (longest expected solves first), so a slow model occupies its own
+//     CTAs instead of keeping the grid in its loop.
+// Measured, grid-wide kernel -> this one, PCG per iteration: 40x10x10 hex beam
+// 5.2 -> 2.7 us, 90-row beam 4.5 -> 1.3, 1,958-row quadratic beam 6.9 -> 2.2,
+// 2,376-row NODAL block 9.4 -> 4.3, 60x30x30 NODAL block 43 -> 15 (FP64) and 36
+// -> 14 (mixed); 256 uneven beams 11.5 -> 2.4 ms per solve.
 // The recurrences, tests, restarts and results are those of pcg.cu's kernel
 // (pipelined CG of Ghysels & Vanroose 2014, then classic PCG after a
 // residual replacement); sums are formed in a fixed order, so results are
-// bit-reproducible and a model's result does not depend on the rest of the
-// pack.
+// bit-reproducible whatever the order in which teams form.  The size of a
+// model's team goes by the pack's models: alone and packed it agrees to
+// rounding.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -52,7 +57,6 @@ constexpr int kRowThreads = kRowWarps * 32;
 // shuffles), in up to kMaxSets sets of kSetRows rows.
 constexpr int kSetRows = kRowWarps * 10;
 constexpr int kMaxSets = 3;
-constexpr int kTeamMaxRows = kSetRows * kMaxSets;
 // steps of a lane's first row group whose blocks stay in its registers
 __host__ __device__ constexpr int reg_blocks(int sets, bool dil) { return sets == 1 ? (dil ? 1 : 2) : 0; }
 constexpr int kWantRows = 46, kWantTeam = 80, kAloneRows = 96;  // see plan_team
