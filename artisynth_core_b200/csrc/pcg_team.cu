@@ -265,14 +265,19 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
   __shared__ TeamSlot s_slot;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const bool red = warp == kRowWarps;
-  // an error of an earlier launch of the call: nothing runs
-  if (*(volatile int*)a.flags != 0) return;
   if (t == 0) s_abort = 0;
 
-  for (;;) {
+  for (bool start = true;; start = false) {
     // next slot; a launch draws n_slots + gridDim tickets in all (one past
-    // the end per CTA), so the counter needs no reset between launches
-    if (t == 0) s_ticket = (int)(atomicAdd(a.ticket, 1ull) % ((unsigned long long)a.n_slots + gridDim.x));
+    // the end per CTA), so the counter needs no reset between launches.
+    // After an error of an earlier launch of the call nothing runs.  One
+    // thread reads the error word and all go by its ticket: other CTAs write
+    // the word while this one starts, and a CTA whose warps saw different
+    // values would wait for those that have left.
+    if (t == 0)
+      s_ticket = start && *(volatile int*)a.flags != 0
+                     ? a.n_slots
+                     : (int)(atomicAdd(a.ticket, 1ull) % ((unsigned long long)a.n_slots + gridDim.x));
     __syncthreads();
     const int si = s_ticket;
     __syncthreads();

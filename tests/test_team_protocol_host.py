@@ -1,0 +1,95 @@
+"""The team PCG kernel (csrc/pcg_team.cu) on the CPU: its source, compiled for
+the host, runs in an emulator of CTAs (tests/emu) that chooses the
+interleaving.  Solves of the layouts that a small GPU test does not reach are
+checked against the residual formed in double; the waits of the error and
+restart paths are checked on the interleavings that a GPU takes once in a very
+long time, where a wait that nothing ends is reported as a hang."""
+import os
+import re
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+EMU = os.path.join(ROOT, "tests", "emu")
+CSRC = os.path.join(ROOT, "artisynth_core_b200", "csrc")
+CUDA_INC = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+
+
+def _without_function(src, head):
+    """src without the function whose definition starts with `head`."""
+    a = src.index(head)
+    i = src.index("{", a)
+    depth = 0
+    while True:
+        depth += {"{": 1, "}": -1}.get(src[i], 0)
+        i += 1
+        if depth == 0:
+            return src[:a] + src[i:]
+
+
+def kernel_source(path=os.path.join(CSRC, "pcg_team.cu")):
+    """The planner and the kernel for the host: the helpers that are inline PTX
+    come from the emulator, shared variables from the running CTA."""
+    src = open(path).read()
+    src = src[:src.index("static std::mutex g_team_mu;")] + "}  // namespace b200fem\n"
+    for head in ("__device__ __forceinline__ void put_packet(", "__device__ __forceinline__ double get_packet(",
+                 "__device__ __forceinline__ unsigned long long team_ns(", "__device__ __forceinline__ void row_barrier("):
+        src = _without_function(src, head)
+    src = src.replace("extern __shared__ __align__(16) unsigned char dyn[];", "unsigned char* const dyn = emu::dyn();")
+
+    def shared(m):
+        out = []
+        for var in m.group(2).split(","):
+            name, dims = re.match(r"\s*(\w+)((?:\[\w+\])*)", var).groups()
+            t = m.group(1) + dims
+            out.append(f"auto& {name} = emu::shared<{t}>(\"{name}\");")
+        return " ".join(out)
+
+    src = re.sub(r"__shared__ (\w+) ([^;]+);", shared, src)
+    assert "__shared__" not in src and "asm" not in re.sub(r"//.*", "", src)
+    return src
+
+
+def build(tmp, path=None):
+    with open(os.path.join(tmp, "team_kernel.inc"), "w") as f:
+        f.write(kernel_source(path) if path else kernel_source())
+    exe = os.path.join(tmp, "team_emu")
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-w", "-pthread", "-I", str(tmp), "-I", EMU, "-I", CSRC, "-I", CUDA_INC,
+                        os.path.join(EMU, "team_emu.cpp"), "-o", exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-4000:]
+    return exe
+
+
+@pytest.fixture(scope="module")
+def emu(tmp_path_factory):
+    exe = build(str(tmp_path_factory.mktemp("emu")))
+
+    def run(*args):
+        r = subprocess.run([exe, *map(str, args)], capture_output=True, text=True, timeout=600)
+        assert r.returncode == 0, (r.returncode, r.stderr)
+        return dict(line.split(" ", 1) for line in r.stdout.splitlines())
+
+    return run
+
+
+SOLVES = {  # grids, stiffness, dil, fp32, CTAs, shared memory KB, variant, what the plan has to show
+    "one_cta": ("4x3x3", "30", 0, 0, 1, 227, 0, {"sets": "1", "team": "1"}),
+}
+
+
+@pytest.mark.parametrize("name", list(SOLVES))
+def test_solves(name, emu):
+    grids, stiff, dil, fp32, ctas, kb, variant, shows = SOLVES[name]
+    out = emu("solve", grids, stiff, 1e-9, dil, fp32, ctas, kb, variant)
+    assert out["ended"] == "yes" and out["flag"] == "0" and out["converged"] == "1", out
+    # the kernel accepts a true residual of at most tol; forming it again in another order moves it by rounding only
+    assert float(out["residual"]) <= 1e-9 * (1 + 1e-3), out
+    assert shows.items() <= out.items(), out
+
+
+@pytest.mark.parametrize("warp", [0, 1, 7, 15])
+def test_error_recorded_while_a_cta_starts(warp, emu):
+    """The CTA's threads leave together or run together, whichever of its warps could see the error first."""
+    out = emu("late_flag", warp)
+    assert out["ended"] == "yes", out
