@@ -354,7 +354,9 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
     // Two roles with the same sequence of CTA barriers per phase: B ends the
     // SpMV and makes the scalars known, C hands the per-warp dot products to
     // the reducing warp, D (classic PCG, true residual) makes a scalar known
-    // that depends on C's.
+    // that depends on C's.  E follows where a role would otherwise go on to
+    // write what the other may not have read yet: the reducing warp s_code
+    // of a restart's first iteration.
     if (red) {
       double sums[3] = {0, 0, 0};
       unsigned pe = 0;  // partial sums published
@@ -446,7 +448,9 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
         if (classic) {
           norms();
           rho = sums[1];
-          conv = sums[2] <= thr2 || sums[2] == 0.0;
+          // (on a restart the residual has just missed the tolerance, though
+          // its square may round to thr2: an iteration is due)
+          conv = restart == 0 && (sums[2] <= thr2 || sums[2] == 0.0);
           first = true;
           for (int it = 0;; it++) {
             if (it > 0) {
@@ -489,7 +493,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
           for (int it = 0;; it++) {
             collect();
             const double gam = sums[0], del = sums[1], rr = sums[2];
-            conv = rr <= thr2 || rr == 0.0;
+            conv = (it > 0 || restart == 0) && (rr <= thr2 || rr == 0.0);
             const int code = conv ? kConverged
                              : (total_it + it >= a.max_iter || (a.variant == 0 && it >= kTeamRoundCap)) ? kStop
                                                                                                        : kRun;
@@ -532,6 +536,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
         __syncthreads();  // D
         if (s_abort) return;
         if (!again) break;
+        __syncthreads();  // E
         if (a.variant == 0) classic = true;
       }
       if (lane == 0 && sl.rank == 0) {
@@ -1050,6 +1055,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
         __syncthreads();  // D
         if (s_abort) return;
         if (s_code != kRun) break;
+        __syncthreads();  // E
         if (a.variant == 0) classic = true;
       }
 #pragma unroll

@@ -275,9 +275,29 @@ static int scenario_late_flag(char** v) {
   return 0;
 }
 
+// The true residual misses a tolerance one unit in the last place below it, so
+// the solve restarts, and its squared form may already meet it; warp 14 is the
+// last to read the verdict: "restart <seed>"
+static int scenario_restart(char** v) {
+  const unsigned seed = (unsigned)atoi(v[0]);
+  double rel = 0;
+  for (int run = 0; run < 2; run++) {
+    Problem P;
+    make(P, {{2, 1, 1}}, {1.0}, run ? std::nextafter(rel, 0.0) : 1e-12, false, seed);
+    if (!plan(P, 1, false)) return 2;
+    emu::Machine m;
+    if (run) m.rank = [](const emu::Fiber& f) { return f.warp() == 14 ? 0 : 1; };
+    const std::string hang = launch(P, m);
+    rel = P.out[1];
+    if (run) report(P, hang);
+  }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   if (s == "solve" && argc == 10) return scenario_solve(argv + 2);
   if (s == "late_flag" && argc == 3) return scenario_late_flag(argv + 2);
+  if (s == "restart" && argc == 3) return scenario_restart(argv + 2);
   return 2;
 }

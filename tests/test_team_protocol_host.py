@@ -93,3 +93,12 @@ def test_error_recorded_while_a_cta_starts(warp, emu):
     """The CTA's threads leave together or run together, whichever of its warps could see the error first."""
     out = emu("late_flag", warp)
     assert out["ended"] == "yes", out
+
+
+@pytest.mark.parametrize("seed", [0, 3, 29, 47])
+def test_restart_within_rounding_of_the_tolerance(seed, emu):
+    """The verdict on the true residual is read by every warp before the restart writes its first code, and the restart
+    iterates even where the square of the residual rounds to the threshold (seeds 3 and 47)."""
+    out = emu("restart", seed)
+    assert out["ended"] == "yes" and out["flag"] == "0" and out["converged"] == "1", out
+    assert float(out["residual"]) <= 1e-12, out
