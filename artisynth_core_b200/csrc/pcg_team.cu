@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
     // the reducing warp, D (classic PCG, true residual) makes a scalar known
     // that depends on C's.  E follows where a role would otherwise go on to
     // write what the other may not have read yet: the reducing warp s_code
-    // of a restart's first iteration.
+    // of a restart's first iteration, a row warp s_abort in its next poll.
     if (red) {
       double sums[3] = {0, 0, 0};
       unsigned pe = 0;  // partial sums published
@@ -520,6 +520,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
             publish();
           }
         }
+        __syncthreads();  // E
         __syncthreads();  // B of the true residual
         if (s_abort) return;
         __syncthreads();  // C
@@ -1033,6 +1034,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
         }
         // ---- the true residual decides; on a miss the recurrences restart
         // from it
+        __syncthreads();  // E
         publish_rows(x);
         poll_rows();
         product();

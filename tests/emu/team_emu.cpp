@@ -294,10 +294,32 @@ static int scenario_restart(char** v) {
   return 0;
 }
 
+// A team of two converges; another model's error is recorded then, CTA 1 is
+// slow to go on and warp 14 of CTA 0 the last of its warps to look at the
+// outcome of the iteration: "slow_warp <variant>"
+static int scenario_slow_warp(char** v) {
+  Problem P;
+  make(P, {{6, 6, 6}}, {1.0}, 1e-6, false, 7);
+  if (!plan(P, 2, false)) return 2;
+  P.a.variant = atoi(v[0]);
+  emu::Machine m;
+  m.before = [&](emu::Fiber&) {
+    auto& s = m.ctas[0]->shared["s_code"];
+    if (P.flags[0] == 0 && !s.empty() && *(int*)(((uintptr_t)s.data() + 15) & ~(uintptr_t)15) != kRun)
+      P.flags[0] = B200FEM_ERR_INVALID_ARG;
+  };
+  m.rank = [&](const emu::Fiber& f) {
+    return P.flags[0] != 0 && (f.cta->block == 1 || f.warp() == 14) ? 0 : 1;
+  };
+  report(P, launch(P, m));
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   if (s == "solve" && argc == 10) return scenario_solve(argv + 2);
   if (s == "late_flag" && argc == 3) return scenario_late_flag(argv + 2);
   if (s == "restart" && argc == 3) return scenario_restart(argv + 2);
+  if (s == "slow_warp" && argc == 3) return scenario_slow_warp(argv + 2);
   return 2;
 }

@@ -102,3 +102,10 @@ def test_restart_within_rounding_of_the_tolerance(seed, emu):
     out = emu("restart", seed)
     assert out["ended"] == "yes" and out["flag"] == "0" and out["converged"] == "1", out
     assert float(out["residual"]) <= 1e-12, out
+
+
+@pytest.mark.parametrize("variant", [0, 1, 2])
+def test_error_recorded_while_a_warp_lags(variant, emu):
+    """A poll that gives up after the last iteration does not take a slower warp out of the loop by another way."""
+    out = emu("slow_warp", variant)
+    assert out["ended"] == "yes" and out["team"] == "2" and out["flag"] != "0", out
