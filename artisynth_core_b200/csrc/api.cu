@@ -1935,7 +1935,7 @@ static int read_step_status(Engine& eng, b200fem_stats* stats, int max_iter, boo
   eng.last_stats = st;
   if (stats) *stats = st;
   if (flags[0] != 0) CK(team_recover(eng));
-  if (flags[0] == B200FEM_ERR_TIMEOUT) return fail(&eng, B200FEM_ERR_TIMEOUT, "PCG grid barrier timed out");
+  if (flags[0] == B200FEM_ERR_TIMEOUT) return fail(&eng, B200FEM_ERR_TIMEOUT, "a wait between the PCG's CTAs timed out");
   if (flags[0] != 0) return fail(&eng, flags[0], "singular diagonal block in the solve matrix");
   if (flags[2] != 0 || !all_conv) {
     char buf[160];

@@ -133,20 +133,34 @@ __device__ __forceinline__ unsigned long long team_ns() {
 }
 
 // The bound of a poll: every 64 tries the wait ends when another CTA has
-// recorded an error or the time limit (counted from the first such check)
-// has passed; the latter records B200FEM_ERR_TIMEOUT.
+// recorded an error or the time limit has passed; the latter records
+// B200FEM_ERR_TIMEOUT.  The limit is for waits between running CTAs, so it
+// counts from the first check that finds the team complete: its first members
+// may have to wait until other CTAs end whole solves of earlier models.  That
+// wait ends with those solves, whose own waits are limited (teams form in
+// ticket order, so only the last one is incomplete); kFormNs bounds it should
+// a CTA be lost.
+constexpr unsigned long long kFormNs = 60000000000ull;
 struct PollBound {
-  int* flags;
-  unsigned long long limit, t0 = 0;
+  const TeamArgs& a;
+  const TeamSlot& sl;
+  const uint64_t& ticket0;  // the launch's first ticket
+  unsigned long long t0 = 0;
   unsigned n = 0;
-  __device__ __forceinline__ PollBound(int* f, unsigned long long l) : flags(f), limit(l) {}
+  bool formed = false;
+  __device__ __forceinline__ PollBound(const TeamArgs& a, const TeamSlot& sl, const uint64_t& ticket0)
+      : a(a), sl(sl), ticket0(ticket0) {}
   __device__ __forceinline__ bool give_up() {
     if ((++n & 63u) != 0) return false;
-    if (*(volatile int*)flags != 0) return true;
+    if (*(volatile int*)a.flags != 0) return true;
     const unsigned long long now = team_ns();
-    if (t0 == 0) t0 = now;
-    else if (now - t0 > limit) {
-      atomicExch(flags, B200FEM_ERR_TIMEOUT);
+    if (!formed && *(volatile unsigned long long*)a.ticket - ticket0 >= (unsigned long long)(sl.s0 + sl.k)) {
+      formed = true;
+      t0 = now;
+    } else if (t0 == 0) {
+      t0 = now;
+    } else if (now - t0 > (formed ? a.timeout_ns : kFormNs)) {
+      atomicExch(a.flags, B200FEM_ERR_TIMEOUT);
       return true;
     }
     return false;
@@ -262,6 +276,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
   __shared__ double s_al, s_be;
   __shared__ int s_code, s_abort;
   __shared__ int s_ticket;
+  __shared__ uint64_t s_ticket0;  // the launch's first ticket
   __shared__ TeamSlot s_slot;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const bool red = warp == kRowWarps;
@@ -274,10 +289,14 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
     // thread reads the error word and all go by its ticket: other CTAs write
     // the word while this one starts, and a CTA whose warps saw different
     // values would wait for those that have left.
-    if (t == 0)
-      s_ticket = start && *(volatile int*)a.flags != 0
-                     ? a.n_slots
-                     : (int)(atomicAdd(a.ticket, 1ull) % ((unsigned long long)a.n_slots + gridDim.x));
+    if (t == 0) {
+      s_ticket = a.n_slots;
+      if (!start || *(volatile int*)a.flags == 0) {
+        const unsigned long long drawn = atomicAdd(a.ticket, 1ull);
+        s_ticket = (int)(drawn % ((unsigned long long)a.n_slots + gridDim.x));
+        s_ticket0 = drawn - s_ticket;
+      }
+    }
     __syncthreads();
     const int si = s_ticket;
     __syncthreads();
@@ -343,7 +362,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
       // failure-detection test: this CTA never publishes; it waits for
       // itself, bounded like every other wait, and the team's waits run out
       if (t == 0) {
-        PollBound pb(a.flags, a.timeout_ns);
+        PollBound pb(a, sl, s_ticket0);
         while (!pb.give_up()) {
         }
       }
@@ -385,7 +404,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
         if (k == 1) return;
         const double* buf = a.part_pk + ((size_t)((pe - 1) & 1) * a.n_slots + sl.s0) * 4 + 2 * (lane & 1);
         const unsigned tag = tag0 + pe;
-        PollBound pb(a.flags, a.timeout_ns);
+        PollBound pb(a, sl, s_ticket0);
         double m = 0, r = 0;
         auto round = [&](auto width, int qb) {
           constexpr int U = decltype(width)::value;
@@ -557,7 +576,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
       auto poll_rows = [&]() {
         const double* buf = a.row_pk + (size_t)((e - 1) & 1) * a.n_rows * 4 + 2 * (t & 1);
         const unsigned tag = tag0 + e;
-        PollBound pb(a.flags, a.timeout_ns);
+        PollBound pb(a, sl, s_ticket0);
         for (int h = t >> 1; h < nh; h += kRowThreads / 2) {
           const double* src = buf + (size_t)hrow[h] * 4;
           unsigned g, hf;
@@ -736,7 +755,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) pcg_team_kernel(TeamArgs a) {
           // t of the neighbours, then each row adds sum_j t_j d_j(row)
           const double* buf = a.t_pk + (size_t)(te & 1) * a.n_rows * 2;
           const unsigned tag = tag0 + te + 1;
-          PollBound pb(a.flags, a.timeout_ns);
+          PollBound pb(a, sl, s_ticket0);
           for (int h = t; h < nh; h += kRowThreads) {
             const double* src = buf + (size_t)hrow[h] * 2;
             unsigned g, hf;

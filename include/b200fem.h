@@ -358,13 +358,18 @@ int b200fem_memory_usage(b200fem_handle h, unsigned long long* bytes);
                                         path avoids the element blocks' HBM round trip but
                                         recomputes boundary elements; it measured slower on the
                                         benchmark meshes and is kept for larger chunks later. */
-#define B200FEM_OPT_BARRIER_TIMEOUT_MS 9 /* bound of every wait at the PCG's grid barriers, in ms
-                                          (1..60000, default 5000): a wait that runs out ends
+#define B200FEM_OPT_BARRIER_TIMEOUT_MS 9 /* bound of every wait of the PCG's CTAs for one another,
+                                          in ms (1..60000, default 5000): at a grid barrier, or
+                                          for the packets of the other CTAs of a complete team
+                                          (the time in which a team's first CTAs wait for those
+                                          that still solve other models does not count; it has a
+                                          bound of its own, a minute).  A wait that runs out ends
                                           the solve with B200FEM_ERR_TIMEOUT and the device
                                           context stays usable (may be changed after the build) */
 #define B200FEM_OPT_TEST_SKIP_ARRIVAL 10 /* failure-detection tests only: CTA index + 1 of the PCG
-                                           kernel that does not arrive at its first grid barrier,
-                                           so every wait there runs out after
+                                           kernel that does not arrive at its first grid barrier
+                                           or, in the team kernel, publishes nothing, so every
+                                           wait for it runs out after
                                            B200FEM_OPT_BARRIER_TIMEOUT_MS; 0 (default) off */
 #define B200FEM_OPT_TET_ASSEMBLY 11 /* BackwardEuler assembly of tetrahedral packs with non-linear
                                        materials: 0 node-row kernel -- a warp per few block rows

@@ -65,6 +65,8 @@ struct Machine {
   // can (0), by choice (1: default)
   std::function<void(Fiber&)> before;
   std::function<int(const Fiber&)> rank = [](const Fiber&) { return 1; };
+  // which of n ready fibers runs next (default: the one that has waited longest)
+  std::function<size_t(size_t n)> choose;
 };
 inline Machine* M = nullptr;
 
@@ -203,6 +205,7 @@ inline std::string run(Machine& m, int grid, int threads, size_t dyn_bytes, std:
     // first come first served; a fiber of rank 0 waits while another can run
     // (a fiber that polls counts as running)
     auto pick = m.ready.begin();
+    if (m.choose) std::swap(*pick, m.ready[m.choose(m.ready.size())]);
     while (pick != m.ready.end() && m.rank(**pick) == 0) ++pick;
     if (pick == m.ready.end()) pick = m.ready.begin();
     Fiber* f = *pick;

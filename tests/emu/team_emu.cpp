@@ -315,11 +315,53 @@ static int scenario_slow_warp(char** v) {
   return 0;
 }
 
+// Two models, three CTAs, a random interleaving; an error is recorded after
+// `at` scheduling steps (0: never): "random <seed> <at> <variant> <dil>"
+static int scenario_random(char** v) {
+  Problem P;
+  const unsigned seed = (unsigned)atoi(v[0]);
+  const long at = atol(v[1]);
+  make(P, {{9, 6, 5}, {3, 2, 2}, {4, 3, 3}}, {4.0, 1.0, 2.0}, 1e-6, atoi(v[3]) != 0, seed);
+  if (!plan(P, 3, false)) return 2;
+  P.a.variant = atoi(v[2]);
+  std::mt19937 rng(seed);
+  emu::Machine m;
+  // runs of one fiber's neighbours, then a jump: warps drift far apart
+  m.choose = [&](size_t n) { return rng() % 8 ? 0 : rng() % n; };
+  m.before = [&](emu::Fiber&) {
+    if (at > 0 && (long)m.resumes >= at) P.flags[0] = B200FEM_ERR_INVALID_ARG;
+  };
+  report(P, launch(P, m));
+  return 0;
+}
+
+// Two CTAs: the first members of a team of two wait until the other CTA ends a
+// long solve of another model.  A scheduling step takes 10 ns, the limit of a
+// wait is 1 ms: "queue"; "queue gone": the second member never publishes.
+static int scenario_queue(bool gone) {
+  Problem P;
+  make(P, {{5, 4, 4}, {5, 4, 4}, {9, 6, 5}}, {100.0, 0.01, 1.0}, 1e-8, false, 7);
+  P.eng.models[1].mat_params[0] = P.eng.models[0].mat_params[0] = 1e6;  // queued first
+  if (!plan(P, 2, false)) return 2;
+  P.a.timeout_ns = 1000000;
+  emu::Machine m;
+  if (gone)  // (its packets are lost)
+    m.before = [&](emu::Fiber&) {
+      for (const TeamSlot& s : P.th.slots)
+        if (s.rank == 1) P.part_pk[4 * (s.s0 + 1) + 1] = P.part_pk[4 * (P.th.slots.size() + s.s0 + 1) + 1] = 0;
+    };
+  report(P, launch(P, m));
+  printf("clock_us %llu\n", (unsigned long long)(m.clock_ns / 1000));
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   if (s == "solve" && argc == 10) return scenario_solve(argv + 2);
   if (s == "late_flag" && argc == 3) return scenario_late_flag(argv + 2);
   if (s == "restart" && argc == 3) return scenario_restart(argv + 2);
   if (s == "slow_warp" && argc == 3) return scenario_slow_warp(argv + 2);
+  if (s == "random" && argc == 6) return scenario_random(argv + 2);
+  if (s == "queue") return scenario_queue(argc == 3);
   return 2;
 }

@@ -154,3 +154,19 @@ def test_missing_member_times_out_and_recovers(skip, b200):
     ref.setState(x, v)
     MechSystemSolver(ref, tol=1e-12).backwardEuler(wl.h, 2)
     assert all(np.array_equal(a, b) for a, b in zip(m.getState(), ref.getState()))
+
+
+def test_short_wait_limit_with_queued_teams(b200):
+    """A limit of 1 ms bounds waits within a team, not the wait for CTAs that solve other models: packs that queue for
+    two CTAs step as with the default limit."""
+    wls = [_beam(L.ELEM_TET, c, NeoHookeanMaterial(E, 0.4))
+           for c, E in (((9, 4, 4), 1e9), ((9, 4, 4), 1e9), ((9, 5, 5), 1e3), ((6, 3, 3), 1e8))]
+    xs, vs = zip(*(_state(w) for w in wls))
+    out = []
+    for ms in (1, 5000):
+        p = FemPack([w.model() for w in wls], precision=L.PREC_FP64,
+                    options={L.OPT_PCG_CTAS: 2, L.OPT_BARRIER_TIMEOUT_MS: ms})
+        p.setStates(xs, vs)
+        p.backwardEuler(wls[0].h, 2, tol=1e-12, max_iter=20000)
+        out.append(p.getStates())
+    assert all(np.array_equal(a, b) for s, t in zip(*out) for a, b in zip(s, t))

@@ -10,6 +10,8 @@ import subprocess
 
 import pytest
 
+from artisynth_core_b200 import _lib as L
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 EMU = os.path.join(ROOT, "tests", "emu")
 CSRC = os.path.join(ROOT, "artisynth_core_b200", "csrc")
@@ -102,6 +104,28 @@ def test_restart_within_rounding_of_the_tolerance(seed, emu):
     out = emu("restart", seed)
     assert out["ended"] == "yes" and out["flag"] == "0" and out["converged"] == "1", out
     assert float(out["residual"]) <= 1e-12, out
+
+
+def test_queueing_for_a_team_is_no_timeout(emu):
+    """The first member of a team waits for the CTA that solves another model for 16 ms with a limit of 1 ms."""
+    out = emu("queue")
+    assert out["ended"] == "yes" and out["flag"] == "0" and out["converged"] == "1", out
+    assert float(out["residual"]) <= 1e-8 * (1 + 1e-3) and int(out["clock_us"]) >= 10000, out
+
+
+def test_lost_packets_of_a_complete_team_time_out(emu):
+    out = emu("queue", "gone")
+    assert out["ended"] == "yes" and out["flag"] == str(L.ERR_TIMEOUT), out
+
+
+@pytest.mark.parametrize("seed", [0, 1, 2, 5])
+@pytest.mark.parametrize("at", [0, 100000])
+def test_random_interleavings(seed, at, emu):
+    """Three models on three CTAs, with and without an error recorded on the way: every thread ends."""
+    out = emu("random", seed, at, seed % 3, seed // 3)
+    assert out["ended"] == "yes", out
+    if at == 0:
+        assert out["flag"] == "0" and float(out["residual"]) <= 1e-6 * (1 + 1e-3), out
 
 
 @pytest.mark.parametrize("variant", [0, 1, 2])
