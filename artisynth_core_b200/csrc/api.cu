@@ -3,20 +3,17 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cfloat>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
-#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <numeric>
 #include <string>
-#include <system_error>
-#include <thread>
 
 #include "engine.h"
+#include "host_stage.h"
 
 namespace b200fem {
 
@@ -1052,180 +1049,9 @@ int build_pack(Engine& eng) {
 
 using namespace b200fem;
 
-namespace {
-// true when every value is finite: a NaN or an infinity in a caller's array
-// is refused with B200FEM_ERR_INVALID_ARG before it reaches the device
-// A double is finite iff its exponent field is not all ones: adding one to
-// the masked exponent carries into bit 63 exactly for all-ones fields.  The
-// OR-reduction vectorises (the host-state step checks 2 x 3N values per
-// call: 9 us for the 40x10x10 hex beam's x or v with a per-element fabs
-// compare, 3 us this way).
-__attribute__((optimize("O3"))) bool all_finite(const double* a, size_t n) {
-  const uint64_t kExp = 0x7ff0000000000000ull, kOne = 0x0010000000000000ull;
-  uint64_t acc = 0;
-  for (size_t i = 0; i < n; i++) {
-    uint64_t b;
-    std::memcpy(&b, a + i, sizeof b);
-    acc |= (b & kExp) + kOne;
-  }
-  return (acc >> 63) == 0;
-}
-}  // namespace
-
 struct b200fem_engine {
   Engine eng;
 };
-
-// Page-locked chunks and a stream for each worker of a staged copy.  The
-// engines of a device share one: page-locking 4 MB takes 5 ms, more than the
-// copies it serves.  It is made on the first staged copy and goes with the
-// last engine that has made one; a copy holds its mutex, so engines in
-// several threads take turns.
-namespace b200fem {
-struct HostStage {
-  static constexpr int kWorkers = 4;
-  static constexpr size_t kChunk = 1 << 20;
-  int device = 0;
-  std::mutex busy;
-  unsigned char* buf = nullptr;
-  cudaStream_t stream[kWorkers] = {};
-  ~HostStage() {
-    cudaSetDevice(device);
-    for (auto& st : stream)
-      if (st) cudaStreamDestroy(st);
-    if (buf) cudaFreeHost(buf);
-  }
-};
-}  // namespace b200fem
-
-namespace {
-// The device's stage, or null with the error that kept it from being made.
-std::shared_ptr<HostStage> host_stage(int device, cudaError_t* err) {
-  static std::mutex mu;
-  static std::map<int, std::weak_ptr<HostStage>> stages;
-  std::lock_guard<std::mutex> lk(mu);
-  std::shared_ptr<HostStage> s = stages[device].lock();
-  if (s) return s;
-  s = std::make_shared<HostStage>();
-  s->device = device;
-  *err = cudaHostAlloc((void**)&s->buf, HostStage::kWorkers * HostStage::kChunk, cudaHostAllocDefault);
-  for (auto& st : s->stream)
-    if (*err == cudaSuccess) *err = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-  if (*err != cudaSuccess) return nullptr;
-  stages[device] = s;
-  return s;
-}
-
-// One array of a host copy.
-struct HostCopy {
-  void* host;
-  void* dev;
-  size_t bytes;
-};
-
-// f(worker) on the stage's number of threads, the caller's among them.
-template <typename F>
-void on_stage_workers(F&& f) {
-  std::vector<std::thread> pool;
-  try {
-    for (int w = 1; w < HostStage::kWorkers; w++) pool.emplace_back(f, w);
-  } catch (const std::system_error&) {  // no more threads: those there are share the work
-  }
-  f(0);
-  for (auto& t : pool) t.join();
-}
-
-bool all_finite_arrays(std::initializer_list<std::pair<const double*, size_t>> arrays) {
-  size_t total = 0;
-  for (auto& a : arrays) total += a.first ? a.second : 0;
-  constexpr size_t kPart = 1 << 17;
-  if (total < 2 * kPart) {
-    for (auto& a : arrays)
-      if (a.first && !all_finite(a.first, a.second)) return false;
-    return true;
-  }
-  std::atomic<size_t> next(0);
-  std::atomic<bool> ok(true);
-  on_stage_workers([&](int) {
-    for (size_t q; ok && (q = next++ * kPart) < total;) {
-      // part [q, q + kPart) of the arrays laid end to end
-      size_t off = q, left = std::min(kPart, total - q);
-      for (auto& a : arrays) {
-        const size_t n = a.first ? a.second : 0;
-        if (off >= n) {
-          off -= n;
-          continue;
-        }
-        const size_t m = std::min(left, n - off);
-        if (!all_finite(a.first + off, m)) ok = false;
-        left -= m;
-        off = 0;
-        if (left == 0) break;
-      }
-    }
-  });
-  return ok;
-}
-
-// Copies between host arrays and the device.  Large pageable arrays go
-// through page-locked chunks, several host threads copying while the DMA
-// engine moves the other chunks: the driver's own staging is one thread, and
-// a destination the caller has just allocated takes its page faults in it
-// (256 beams of 331,000 nodes, set, step and get: 11.6 ms, 8.5 this way and with
-// the velocity history copied on the device).
-// Small or page-locked arrays take plain asynchronous copies on the engine's
-// stream.  Staged copies are complete on return; either way the caller
-// synchronises the stream before it reads.
-// (kStageMin: an update's 16 MB take 2.2 ms staged and 3.6 plain, 4 MB 1.4 and
-// 1.2: below it the threads cost more than they save)
-constexpr size_t kStageMin = 6 << 20;
-cudaError_t stage_copy(Engine& eng, std::initializer_list<HostCopy> list, bool to_host) {
-  const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
-  std::vector<HostCopy> chunks;
-  cudaError_t e = cudaSuccess;
-  size_t staged = 0, total = 0;
-  for (const HostCopy& c : list) total += c.host ? c.bytes : 0;
-  for (const HostCopy& c : list) {
-    if (!c.host || c.bytes == 0) continue;
-    bool pageable = total >= kStageMin && c.bytes >= HostStage::kChunk;
-    if (pageable) {
-      cudaPointerAttributes at{};
-      if (cudaPointerGetAttributes(&at, c.host) != cudaSuccess) cudaGetLastError();
-      else pageable = at.type == cudaMemoryTypeUnregistered;
-    }
-    if (!pageable) {
-      e = cudaMemcpyAsync(to_host ? c.host : c.dev, to_host ? c.dev : c.host, c.bytes, kind, eng.stream);
-      if (e != cudaSuccess) return e;
-      continue;
-    }
-    for (size_t o = 0; o < c.bytes; o += HostStage::kChunk)
-      chunks.push_back({(char*)c.host + o, (char*)c.dev + o, std::min(HostStage::kChunk, c.bytes - o)});
-    staged += c.bytes;
-  }
-  if (staged == 0) return cudaSuccess;
-  if (!eng.stage) eng.stage = host_stage(eng.device, &e);
-  if (!eng.stage) return e;
-  HostStage& stage = *eng.stage;
-  std::lock_guard<std::mutex> lk(stage.busy);
-  // earlier work on the engine's stream writes the source or reads the target
-  if ((e = cudaStreamSynchronize(eng.stream)) != cudaSuccess) return e;
-  std::atomic<size_t> next(0);
-  std::atomic<int> err((int)cudaSuccess);
-  on_stage_workers([&](int w) {
-    cudaError_t r = cudaSetDevice(eng.device);
-    unsigned char* buf = stage.buf + (size_t)w * HostStage::kChunk;
-    for (size_t q; r == cudaSuccess && err == (int)cudaSuccess && (q = next++) < chunks.size();) {
-      const HostCopy& c = chunks[q];
-      if (!to_host) std::memcpy(buf, c.host, c.bytes);
-      r = cudaMemcpyAsync(to_host ? (void*)buf : c.dev, to_host ? c.dev : (void*)buf, c.bytes, kind, stage.stream[w]);
-      if (r == cudaSuccess) r = cudaStreamSynchronize(stage.stream[w]);
-      if (r == cudaSuccess && to_host) std::memcpy(c.host, buf, c.bytes);
-    }
-    if (r != cudaSuccess) err = (int)r;
-  });
-  return (cudaError_t)(int)err;
-}
-}  // namespace
 
 #define ENG(h)                                                    \
   if (!(h)) return fail(nullptr, B200FEM_ERR_INVALID_ARG, "null handle"); \
@@ -1813,7 +1639,7 @@ int b200fem_set_state(b200fem_handle h, const double* x, const double* v) {
   size_t n = 3 * (size_t)eng.d.n_nodes * sizeof(double);
   if (!all_finite_arrays({{x, 3 * (size_t)eng.d.n_nodes}, {v, 3 * (size_t)eng.d.n_nodes}}))
     return fail(&eng, B200FEM_ERR_INVALID_ARG, "non-finite position or velocity");
-  CK(stage_copy(eng, {{(void*)x, eng.d.x, n}, {(void*)v, eng.d.v, n}}, false));
+  CK(stage_copy(eng.device, eng.stream, eng.stage, {{(void*)x, eng.d.x, n}, {(void*)v, eng.d.v, n}}, false));
   // a state set from outside has no history: extrapolation starts at zero
   // acceleration (the history is copied on the device, not sent four times)
   if (v)
@@ -1827,7 +1653,7 @@ int b200fem_get_state(b200fem_handle h, double* x, double* v) {
   ENG(h);
   NEED_BUILT();
   size_t n = 3 * (size_t)eng.d.n_nodes * sizeof(double);
-  CK(stage_copy(eng, {{x, eng.d.x, n}, {v, eng.d.v, n}}, true));
+  CK(stage_copy(eng.device, eng.stream, eng.stage, {{x, eng.d.x, n}, {v, eng.d.v, n}}, true));
   CK(cudaStreamSynchronize(eng.stream));
   return B200FEM_OK;
 }
@@ -1872,7 +1698,7 @@ int b200fem_update_stress_stiffness(b200fem_handle h, const double* x, double* f
       crs_export_kernel_launch(eng, nbr, d.red_row, d.red_rowptr, d.K_red, d.crs_red);
       CK(cudaGetLastError());
     }
-    CK(stage_copy(eng,
+    CK(stage_copy(eng.device, eng.stream, eng.stage,
                   {{f_int, d.fint, fbytes},
                    {k_blocks, d.K_red, 9 * sizeof(double) * (size_t)nbr},
                    {crs_vals, d.crs_red, 9 * sizeof(double) * (size_t)nbr}},
@@ -1880,13 +1706,13 @@ int b200fem_update_stress_stiffness(b200fem_handle h, const double* x, double* f
   } else if (crs_vals && !d.S) {
     // mixed form (no FP64 S buffer): permute to the CRS slot order on the host
     kbsr.resize(9 * (size_t)d.nnzb);
-    CK(stage_copy(eng, {{f_int, d.fint, fbytes}, {k_blocks, d.K, kbytes}, {kbsr.data(), d.K, kbytes}}, true));
+    CK(stage_copy(eng.device, eng.stream, eng.stage, {{f_int, d.fint, fbytes}, {k_blocks, d.K, kbytes}, {kbsr.data(), d.K, kbytes}}, true));
   } else {
     if (crs_vals) {
       CK(launch_crs_export(eng, d.K, d.S));
       eng.have_matrix = false;  // S was used as scratch
     }
-    CK(stage_copy(eng, {{f_int, d.fint, fbytes}, {k_blocks, d.K, kbytes}, {crs_vals, d.S, kbytes}}, true));
+    CK(stage_copy(eng.device, eng.stream, eng.stage, {{f_int, d.fint, fbytes}, {k_blocks, d.K, kbytes}, {crs_vals, d.S, kbytes}}, true));
   }
   CK(cudaStreamSynchronize(eng.stream));
   if (!kbsr.empty()) {
