@@ -33,8 +33,9 @@ __attribute__((optimize("O3"))) bool all_finite(const double* a, size_t n) {
 // Page-locked chunks and a stream for each worker of a staged copy.  The
 // engines of a device share one: page-locking 4 MB takes 5 ms, more than the
 // copies it serves.  It is made on the first staged copy and goes with the
-// last engine that has made one; a copy holds its mutex, so engines in
-// several threads take turns.
+// last engine that has made one.  A copy holds its mutex; another engine's
+// copy takes the plain way meanwhile, so engines in several threads do not
+// wait for one another.
 struct HostStage {
   static constexpr int kWorkers = 4;
   static constexpr size_t kChunk = 1 << 20;
@@ -51,11 +52,13 @@ struct HostStage {
 };
 
 namespace {
-// The device's stage, or null where its memory or streams cannot be had.
+// The device's stage, or null where its memory or streams cannot be had (or
+// another thread is making one).
 std::shared_ptr<HostStage> host_stage(int device) {
   static std::mutex mu;
   static std::map<int, std::weak_ptr<HostStage>> stages;
-  std::lock_guard<std::mutex> lk(mu);
+  std::unique_lock<std::mutex> lk(mu, std::try_to_lock);
+  if (!lk) return nullptr;
   std::shared_ptr<HostStage> s = stages[device].lock();
   if (s) return s;
   s = std::make_shared<HostStage>();
@@ -124,7 +127,8 @@ bool all_finite_arrays(std::initializer_list<std::pair<const double*, size_t>> a
 // (256 beams of 331,000 nodes, set, step and get: 11.6 ms, 8.5 this way and with
 // the velocity history copied on the device).
 // Small or page-locked arrays take plain asynchronous copies on the engine's
-// stream, and so do all where the stage cannot be had.
+// stream, and so do all where the stage cannot be had or another engine uses
+// it.
 // (kStageMin: an update's 16 MB take 2.2 ms staged and 3.6 plain, 4 MB 1.4 and
 // 1.2: below it the threads cost more than they save)
 constexpr size_t kStageMin = 6 << 20;
@@ -151,7 +155,14 @@ cudaError_t stage_copy(int device, cudaStream_t stream, std::shared_ptr<HostStag
   }
   if (large.empty()) return cudaSuccess;
   if (!hold) hold = host_stage(device);
-  if (!hold) {
+  std::unique_lock<std::mutex> lk;
+  if (hold) {
+    // earlier work on the engine's stream writes the source or reads the
+    // target; it is awaited before the stage is taken from the others
+    if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return e;
+    lk = std::unique_lock<std::mutex>(hold->busy, std::try_to_lock);
+  }
+  if (!lk.owns_lock()) {
     for (const HostCopy& c : large)
       if ((e = plain(c)) != cudaSuccess) return e;
     return cudaSuccess;
@@ -160,9 +171,6 @@ cudaError_t stage_copy(int device, cudaStream_t stream, std::shared_ptr<HostStag
   for (const HostCopy& c : large)
     for (size_t o = 0; o < c.bytes; o += HostStage::kChunk)
       chunks.push_back({(char*)c.host + o, (char*)c.dev + o, std::min(HostStage::kChunk, c.bytes - o)});
-  std::lock_guard<std::mutex> lk(stage.busy);
-  // earlier work on the engine's stream writes the source or reads the target
-  if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return e;
   std::atomic<size_t> next(0);
   std::atomic<int> err((int)cudaSuccess);
   on_stage_workers([&](int w) {

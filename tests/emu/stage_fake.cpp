@@ -114,5 +114,30 @@ int main(int argc, char** argv) {
     bad += check(c.get(kA) == cudaSuccess && c.same() && g_host_bufs == 1, "no stage later");
     return bad;
   }
+  if (s == "stage_in_use" || s == "stream_busy") {
+    // another engine's copy or earlier work does not end: this one's copy does
+    Copy a((size_t)1 << 20), b((size_t)1 << 20);
+    a.get(kA);
+    std::fill(a.host.begin(), a.host.end(), 0.0);
+    (s == "stage_in_use" ? g_block_stage : g_busy[kA]) = true;
+    std::thread ta([&] { a.get(kA); });
+    while (g_waiting == 0) std::this_thread::yield();
+    std::atomic<bool> done(false);
+    std::thread tb([&] {
+      b.get(kB);
+      done = true;
+    });
+    for (int i = 0; i < 500 && !done; i++) std::this_thread::sleep_for(std::chrono::milliseconds(10));
+    bad += check(done, "waits for the other engine");
+    {
+      std::lock_guard<std::mutex> lk(g_mu);
+      g_block_stage = g_busy[kA] = false;
+    }
+    g_cv.notify_all();
+    ta.join();
+    tb.join();
+    bad += check(a.same() && b.same(), "wrong values");
+    return bad;
+  }
   return 2;
 }

@@ -1,6 +1,6 @@
 """Host copies through the page-locked stage (csrc/host_stage.cpp) against a
 CUDA runtime made of host memory (tests/emu/stage_fake.cpp): what a copy does
-when the stage cannot be had."""
+when the stage cannot be had or another engine holds it up."""
 import os
 import subprocess
 
@@ -21,7 +21,7 @@ def exe(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("scenario", ["no_host_memory", "no_stream"])
+@pytest.mark.parametrize("scenario", ["no_host_memory", "no_stream", "stage_in_use", "stream_busy"])
 def test_copies_without_a_stage(scenario, exe):
     r = subprocess.run([exe, scenario], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout
