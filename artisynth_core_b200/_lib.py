@@ -43,6 +43,7 @@ OPT_PCG_RESIDENT = 12
 OPT_NODAL_FACTORED = 13
 INTEGRATOR_BACKWARD_EULER, INTEGRATOR_CONSTRAINED_BACKWARD_EULER = 0, 1
 SPLIT_AUTO, SPLIT_CONTIGUOUS, SPLIT_STRIDED, SPLIT_CLUSTER = 0, 1, 2, 3
+SPLIT_TEAM = 4  # reported after the build; what auto takes where it applies
 
 
 class B200FemError(RuntimeError):

@@ -9,7 +9,9 @@ What it chooses, by timing real BackwardEuler steps on the device:
                   finely the models are dealt over the CTAs, which sets the
                   PCG schedule of the pack.
 ROW_LANES and ELEM_TILE change on the built pack; PIECE_ROWS needs a build
-per candidate.  The tuning steps run on a copy of the state that is put back
+per candidate.  Where auto runs one team of CTAs per model (PCG_SPLIT reads
+back as 4), the PCG uses neither ROW_LANES nor PIECE_ROWS and only ELEM_TILE
+is timed.  The tuning steps run on a copy of the state that is put back
 afterwards, so tuning leaves the models where they were.
 
 Results are cached by the shape of the pack -- element type and material
@@ -90,8 +92,8 @@ def tune_runtime(pack, h, tol, reps=2):
     xs, vs = [x.copy() for x, _ in saved], [v.copy() for _, v in saved]
     pack.backwardEuler(h, 1, tol=tol)  # warm-up (graph capture)
     timings = {}
-    best_lanes, best_pcg = None, math.inf
-    for lanes in LANES:
+    best_lanes, best_pcg = pack.option(L.OPT_ROW_LANES), math.inf
+    for lanes in LANES if pack.option(L.OPT_PCG_SPLIT) != L.SPLIT_TEAM else ():
         pack.setOption(L.OPT_ROW_LANES, lanes)
         pack.setStates(xs, vs)
         pack.backwardEuler(h, 1, tol=tol)
@@ -99,7 +101,8 @@ def tune_runtime(pack, h, tol, reps=2):
         timings[f"lanes{lanes}_pcg_ms_per_it"] = p
         if p < best_pcg:
             best_lanes, best_pcg = lanes, p
-    pack.setOption(L.OPT_ROW_LANES, best_lanes)
+    if best_pcg < math.inf:
+        pack.setOption(L.OPT_ROW_LANES, best_lanes)
     best_tile, best_asm = None, math.inf
     for tile in TILES:
         pack.setOption(L.OPT_ELEM_TILE, tile)

@@ -1453,7 +1453,7 @@ int b200fem_set_option(b200fem_handle h, int key, int value) {
       eng.opt_row_lanes = value;
       if (eng.built && value != 0 && value != eng.pcg_row_lanes) {
         eng.pcg_row_lanes = value;
-        eng.step_exec_max_iter = -1;  // recapture: the width is a kernel argument
+        if (!eng.team) eng.step_exec_max_iter = -1;  // recapture: the width is a kernel argument
       }
       return B200FEM_OK;
     case B200FEM_OPT_PCG_RESIDENT:
@@ -1495,10 +1495,10 @@ int b200fem_get_option(b200fem_handle h, int key, int* value) {
   if (!value) return fail(&eng, B200FEM_ERR_INVALID_ARG, "null value");
   switch (key) {
     case B200FEM_OPT_PCG_SPLIT:
-      *value = eng.built ? (eng.pcg_cluster ? 3 : eng.pcg_strided ? 2 : 1) : eng.opt_split;
+      *value = eng.built ? (eng.pcg_cluster ? 3 : eng.team ? 4 : eng.pcg_strided ? 2 : 1) : eng.opt_split;
       break;
     case B200FEM_OPT_ROW_LANES: *value = eng.built ? eng.pcg_row_lanes : eng.opt_row_lanes; break;
-    case B200FEM_OPT_PCG_CTAS: *value = eng.built ? eng.pcg_grid : eng.opt_ctas; break;
+    case B200FEM_OPT_PCG_CTAS: *value = eng.built ? (eng.team ? eng.team_grid : eng.pcg_grid) : eng.opt_ctas; break;
     case B200FEM_OPT_PIECE_ROWS: *value = eng.opt_piece_rows; break;
     case B200FEM_OPT_WARM_START: *value = eng.opt_warm_start; break;
     case B200FEM_OPT_ELEM_TILE: *value = eng.elem_staged ? (eng.elem_tile_small ? 2 : 1) : 0; break;

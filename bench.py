@@ -441,7 +441,7 @@ def run_batched(dev, steps=20, tol=1e-10, sample_every=4, tune=True, layout=None
     return {
         "workload": "256 uneven NeoHookean tet beams (n 4-60, m 2-8, seed 3), 20 steps h=0.01",
         "models": n, "tets": int(sum(b.conn.shape[0] for b in bs)), "steps": steps, "tol": tol,
-        "precision": "mixed FP32 element/SpMV, FP64 vectors", "pcg_split": {1: "contiguous", 2: "strided", 3: "cluster"}.get(split, str(split)),
+        "precision": "mixed FP32 element/SpMV, FP64 vectors", "pcg_split": {1: "contiguous", 2: "strided", 3: "cluster", 4: "teams"}.get(split, str(split)),
         "device_bytes": nbytes, "build_and_tune_s": build_s,
         "tuned": {k: v for k, v in tuned.items() if not k.endswith("_ms") and not k.endswith("_it")},
         "model_steps_per_s": n * steps / wall, "device_ms_per_step": (asm + pcg) / steps,

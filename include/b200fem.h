@@ -325,13 +325,16 @@ int b200fem_memory_usage(b200fem_handle h, unsigned long long* bytes);
                                     into short pieces dealt over all CTAs; 3 cluster: one
                                     thread-block cluster per model, models taken from a
                                     queue largest first.  Auto: one team of CTAs per model
-                                    (pcg_team.cu) wherever every model fits one; the split
-                                    reported, and used where one does not, is contiguous
-                                    when the rows fit shared-memory residency or the handle
-                                    has one model, else strided (the 256-beam pack, solve
-                                    per step: teams 2.4 ms, strided 11.5, cluster 14.2) */
-#define B200FEM_OPT_ROW_LANES 2  /* lanes per block row in the iteration SpMV: 0 auto, 4, 8, 16, 32 */
-#define B200FEM_OPT_PCG_CTAS 3   /* CTAs of the persistent PCG kernel: 0 auto (one per SM) */
+                                    (pcg_team.cu) wherever every model fits one; where one
+                                    does not, contiguous when the rows fit shared-memory
+                                    residency or the handle has one model, else strided (the
+                                    256-beam pack, solve per step: teams 2.4 ms, strided
+                                    11.5, cluster 14.2).  After the build it reads back as
+                                    the split in force, 4 for the teams (4 cannot be set) */
+#define B200FEM_OPT_ROW_LANES 2  /* lanes per block row in the iteration SpMV: 0 auto, 4, 8, 16, 32
+                                    (splits 1 and 2; the teams choose lanes row by row) */
+#define B200FEM_OPT_PCG_CTAS 3   /* most CTAs of the persistent PCG kernel: 0 auto (one per SM);
+                                    after the build those it launches */
 #define B200FEM_OPT_PIECE_ROWS 4 /* block rows per piece in the strided split: 0 auto (64) */
 #define B200FEM_OPT_WARM_START 5 /* PCG start: the velocity extrapolated by a polynomial of
                                     order 0..4 through the last 1..5 velocities: 0 v_n; 1

@@ -78,6 +78,29 @@ def test_picks_fastest_and_restores_state(tmp_path):
     assert pack2.opts[L.OPT_ROW_LANES] == 8 and pack2.opts[L.OPT_PIECE_ROWS] == 32
 
 
+class TeamPack(FakePack):
+    """Auto took the team PCG: lanes and pieces change nothing."""
+
+    def option(self, key):
+        return L.SPLIT_TEAM if key == L.OPT_PCG_SPLIT else self.opts[key]
+
+    def setOption(self, key, value):
+        assert key == L.OPT_ELEM_TILE, key
+        super().setOption(key, value)
+
+
+def test_teams_tune_the_element_kernel_only(tmp_path):
+    ms = models()
+    FakePack.built = 0
+    pack, res, hit = autotune.tune_pack(lambda o: TeamPack(ms, o), ms, L.PREC_MIXED, 0.01, 1e-6,
+                                        cache=autotune.TuneCache(str(tmp_path / "tune.json")))
+    assert not hit and FakePack.built == 1
+    assert res["row_lanes"] == 16 and res["elem_tile"] == 2 and "piece_rows" not in res
+    assert not any(k.startswith(("lanes", "piece")) for k in res)
+    for x, v in pack.getStates():
+        assert np.all(v == 0)
+
+
 def test_shape_key_separates_precision_and_size():
     ms = models()
     k1 = autotune.shape_key(ms, L.PREC_MIXED)

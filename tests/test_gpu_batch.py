@@ -194,6 +194,30 @@ def test_row_lanes_change_after_build(beams):
     assert np.all(np.isfinite(np.concatenate([xg for xg, _ in pack.getStates()])))
 
 
+def test_split_in_force_is_reported(beams):
+    """Auto reports the teams it runs and their CTAs; tuning them leaves lanes and pieces alone."""
+    pack = FemPack([b.model() for b in beams], precision=L.PREC_FP64, options={L.OPT_PCG_CTAS: 5})
+    pack.engine()
+    assert pack.option(L.OPT_PCG_SPLIT) == L.SPLIT_TEAM and pack.option(L.OPT_PCG_CTAS) == 5
+    with pytest.raises(L.B200FemError):
+        FemPack([b.model() for b in beams], precision=L.PREC_FP64, options={L.OPT_PCG_SPLIT: L.SPLIT_TEAM}).engine()
+
+
+@pytest.mark.parametrize("split", [L.SPLIT_CONTIGUOUS, L.SPLIT_STRIDED])
+def test_row_lanes_after_build_agree(split, beams):
+    """Every lane width of the grid-wide kernel, changed on the built pack, takes the same step to rounding."""
+    pack = FemPack([b.model() for b in beams], precision=L.PREC_FP64, options={L.OPT_PCG_SPLIT: split})
+    xs, vs = [b.rest for b in beams], [np.zeros_like(b.rest) for b in beams]
+    ref = None
+    for lanes in (4, 8, 16, 32):
+        pack.setOption(L.OPT_ROW_LANES, lanes)
+        pack.setStates(xs, vs)
+        pack.backwardEuler(beams[0].h, 2, tol=1e-12)
+        x = np.concatenate([xg for xg, _ in pack.getStates()])
+        ref = x if ref is None else ref
+        assert rel_err(x, ref) <= 1e-9, lanes
+
+
 def test_autotune_sets_options_and_keeps_results(beams, tmp_path):
     from artisynth_core_b200 import autotune
     models = [b.model() for b in beams]
