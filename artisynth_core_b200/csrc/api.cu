@@ -776,7 +776,7 @@ int build_pack(Engine& eng) {
   // fit the shared memory of the CTAs; the split above serves the rest and
   // the layouts asked for explicitly
   TeamHost team;
-  eng.team = eng.opt_split == 0 && eng.opt_resident != 1 &&
+  eng.team = eng.opt_split == 0 && eng.opt_resident == 0 &&
              plan_team(eng, gmax, prow, eng.factored ? s1_col : col, eng.factored ? s1_diag : blk_diag,
                        eng.factored && !dil_nodes.empty(), team);
 

@@ -388,8 +388,10 @@ int b200fem_memory_usage(b200fem_handle h, unsigned long long* bytes);
                                        when the CTA's rows fit (512-thread CTAs, one per SM); 1
                                        never (1024-thread CTAs, global vectors: twice the warps
                                        for the SpMV's loads); 0 (auto) as 2 while the solve
-                                       matrix is at most 64 MB (it stays in L2), else as 1.  Set
-                                       before b200fem_build; after it, 2 or 1 as in force */
+                                       matrix is at most 64 MB (it stays in L2), else as 1.  1 and
+                                       2 ask for that kernel: auto then takes no teams.  Set
+                                       before b200fem_build; after it, 2 or 1 as in force (or as
+                                       it would be) */
 #define B200FEM_OPT_NODAL_FACTORED 13 /* BackwardEuler solve matrix of NODAL models: 2 factored
                                          -- the element blocks of direct neighbours assembled
                                          (S1), the dilational term (h^2 + h beta) sum_n kp_n

@@ -170,3 +170,18 @@ def test_short_wait_limit_with_queued_teams(b200):
         p.backwardEuler(wls[0].h, 2, tol=1e-12, max_iter=20000)
         out.append(p.getStates())
     assert all(np.array_equal(a, b) for s, t in zip(*out) for a, b in zip(s, t))
+
+
+@pytest.mark.parametrize("resident", [1, 2])
+def test_explicit_residency_keeps_the_grid_wide_kernel(resident, b200):
+    """PCG_RESIDENT asks for a layout of the contiguous split: it is the one that runs."""
+    wl = _beam(L.ELEM_HEX, (8, 4, 4), NH)
+    out = []
+    for opts in ({L.OPT_PCG_RESIDENT: resident}, {L.OPT_PCG_RESIDENT: resident, L.OPT_PCG_SPLIT: L.SPLIT_CONTIGUOUS}):
+        p = FemPack([wl.model()], precision=L.PREC_FP64, options=opts)
+        p.engine()
+        assert p.option(L.OPT_PCG_SPLIT) == L.SPLIT_CONTIGUOUS and p.option(L.OPT_PCG_RESIDENT) == resident
+        p.setStates(*([a] for a in _state(wl)))
+        p.backwardEuler(wl.h, 2, tol=1e-12)
+        out.append(p.getStates()[0])
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
