@@ -7,6 +7,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <future>
 #include <map>
 #include <mutex>
 #include <numeric>
@@ -774,11 +775,14 @@ int build_pack(Engine& eng) {
 
   // ---- one team of CTAs per model (pcg_team.cu) wherever every model's rows
   // fit the shared memory of the CTAs; the split above serves the rest and
-  // the layouts asked for explicitly
+  // the layouts asked for explicitly.  Planned beside the uploads, which do
+  // not depend on it (40x10x10 hex beam: 2 ms beside 4).
   TeamHost team;
-  eng.team = eng.opt_split == 0 && eng.opt_resident == 0 &&
-             plan_team(eng, gmax, prow, eng.factored ? s1_col : col, eng.factored ? s1_diag : blk_diag,
-                       eng.factored && !dil_nodes.empty(), team);
+  std::future<bool> planned = std::async([&] {
+    return eng.opt_split == 0 && eng.opt_resident == 0 &&
+           plan_team(eng, gmax, prow, eng.factored ? s1_col : col, eng.factored ? s1_diag : blk_diag,
+                     eng.factored && !dil_nodes.empty(), team);
+  });
 
   // ---- device upload
   CK(upload(eng, &d.x, x));
@@ -884,9 +888,8 @@ int build_pack(Engine& eng) {
     CK(cudaMemset(d.dil_t, 0, sizeof(double) * (size_t)N));
   }
   CK(dalloc(eng, &d.elemF, (size_t)coff[E] * 3));
-  CK(dalloc(eng, &d.Dinv, (size_t)R * 9));
   CK(dalloc(eng, &d.fint, 3 * (size_t)N));
-  for (double** v : {&d.b, &d.sol, &d.r, &d.z, &d.p, &d.q, &d.w, &d.u, &d.s, &d.m0, &d.m1}) {
+  for (double** v : {&d.b, &d.sol, &d.w, &d.q}) {  // (w and q: b200fem_spmv's too)
     CK(dalloc(eng, v, 3 * (size_t)R));
     CK(cudaMemset(*v, 0, 3 * sizeof(double) * (size_t)R));
   }
@@ -929,14 +932,9 @@ int build_pack(Engine& eng) {
     CK(upload(eng, &d.dil_ptr, dptr));
     CK(upload(eng, &d.dil_idx, didx));
   }
-  CK(dalloc(eng, &d.partials, (size_t)d.n_pieces * 8));
-  CK(upload(eng, &d.piece_row, piece_row));
-  CK(upload(eng, &d.piece_model, piece_model));
-  CK(upload(eng, &d.model_piece, model_piece));
-  CK(upload(eng, &d.cta_piece, cta_piece));
-  CK(upload(eng, &d.cta_plist, cta_plist));
+  d.unconv_cap = 200000;
   CK(upload(eng, &d.model_active, std::vector<int>(M, 1)));
-  {
+  if (eng.pcg_cluster) {
     // cluster split: model rows, the queue order (most blocks first) and the
     // queue counter
     std::vector<int> model_row(eng.row_off.begin(), eng.row_off.end()), order(M);
@@ -949,8 +947,6 @@ int build_pack(Engine& eng) {
     CK(dalloc(eng, &d.cl_queue, 1));
   }
   eng.any_inactive = false;
-  d.unconv_cap = 200000;
-  CK(dalloc(eng, &d.unconv, (size_t)d.unconv_cap + 2));
   {
     // models without active rows never run PCG: report them converged
     std::vector<double> ms((size_t)M * 4, 0.0);
@@ -971,7 +967,25 @@ int build_pack(Engine& eng) {
       CK(upload(eng, &d.model_scal2, ms));
     }
   }
-  if (eng.team) {
+  eng.team = planned.get();
+  if (!eng.team) {
+    // the vectors and lists of the grid-wide and cluster PCG; the teams hold
+    // theirs in registers
+    CK(dalloc(eng, &d.Dinv, (size_t)R * 9));
+    for (double** v : {&d.r, &d.z, &d.p, &d.u, &d.s, &d.m0, &d.m1}) {
+      CK(dalloc(eng, v, 3 * (size_t)R));
+      CK(cudaMemset(*v, 0, 3 * sizeof(double) * (size_t)R));
+    }
+    CK(dalloc(eng, &d.partials, (size_t)d.n_pieces * 8));
+    CK(upload(eng, &d.piece_row, piece_row));
+    CK(upload(eng, &d.piece_model, piece_model));
+    CK(upload(eng, &d.model_piece, model_piece));
+    CK(upload(eng, &d.cta_piece, cta_piece));
+    CK(upload(eng, &d.cta_plist, cta_plist));
+    CK(dalloc(eng, &d.barrier, 2));
+    CK(cudaMemset(d.barrier, 0, 2 * sizeof(unsigned)));
+    CK(dalloc(eng, &d.unconv, (size_t)d.unconv_cap + 2));
+  } else {
     eng.team_grid = team.grid;
     eng.team_smem = team.smem;
     eng.team_sets = team.sets;
@@ -1023,8 +1037,6 @@ int build_pack(Engine& eng) {
       CK(upload(eng, &d.team_g2, g2));
     }
   }
-  CK(dalloc(eng, &d.barrier, 2));
-  CK(cudaMemset(d.barrier, 0, 2 * sizeof(unsigned)));
   CK(dalloc(eng, &d.flags, 4));
   CK(cudaMemset(d.flags, 0, 4 * sizeof(int)));
   CK(dalloc(eng, &d.dmin, 1));

@@ -496,7 +496,7 @@ struct TeamHost {
   int grid = 0, sets = 1, stream = 0, step_bytes = 0;
   size_t smem = 0;
 };
-bool plan_team(Engine& eng, int grid_max, const std::vector<int>& rowptr, const std::vector<int>& col,
+bool plan_team(const Engine& eng, int grid_max, const std::vector<int>& rowptr, const std::vector<int>& col,
                const std::vector<int>& diag, bool dil, TeamHost& out);
 // f(i) for i in [0, n) on the host's threads
 void team_parallel(int n, const std::function<void(int)>& f);

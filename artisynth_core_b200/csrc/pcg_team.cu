@@ -1388,6 +1388,10 @@ static bool team_split_model(int row0, int n, int k, int sets, const std::vector
   if (!fits) return false;
   result = TeamSplit();
   result.pub.assign(n, 0);
+  size_t lanes = 0;
+  for (const TeamSplit& p : piece) lanes += p.cl.size();
+  result.cl.reserve(lanes);
+  result.blk.reserve(lanes);
   for (TeamSplit& p : piece) {
     for (int h : p.halo) result.pub[h - row0] = 1;
     append_split(result, p);
@@ -1416,7 +1420,7 @@ static double expected_iterations(const ModelDesc& m, const ModelHost& h) {
 
 // The team layout of a pack: per model the number of CTAs, its split, and the
 // slots of all models in queue order.
-bool plan_team(Engine& eng, int grid_max, const std::vector<int>& rowptr, const std::vector<int>& col,
+bool plan_team(const Engine& eng, int grid_max, const std::vector<int>& rowptr, const std::vector<int>& col,
                const std::vector<int>& diag, bool dil, TeamHost& out) {
   const int M = (int)eng.hosts.size();
   const int mt = eng.precision == B200FEM_PREC_MIXED ? 4 : 8;
@@ -1518,7 +1522,7 @@ bool plan_team(Engine& eng, int grid_max, const std::vector<int>& rowptr, const 
       // the largest team streams what does not fit
       const bool last = k >= std::min(grid_max, n);
       if (team_split_model(a, n, k, sets, rowptr, col, eng.models[m].rest.data(), eng.hosts[m].act_node.data(), mt,
-                           dil, budget, last, across > 1 ? 1 : std::min(threads, 1 + n / 4096), split[m]))
+                           dil, budget, last, across > 1 ? 1 : std::min(threads, 1 + n / 512), split[m]))
         break;
       if (last) good = false;
     }
@@ -1535,7 +1539,19 @@ bool plan_team(Engine& eng, int grid_max, const std::vector<int>& rowptr, const 
       s.model = m;
       s.s0 = s0;
     }
-    append_split(out, sp);
+    if (order.size() == 1) {
+      // (one model: nothing to shift)
+      out.slots.swap(sp.slots);
+      out.rows.swap(sp.rows);
+      out.halo.swap(sp.halo);
+      out.blk.swap(sp.blk);
+      out.group.swap(sp.group);
+      out.cl.swap(sp.cl);
+      out.smem = sp.smem;
+      out.stream = sp.stream;
+    } else {
+      append_split(out, sp);
+    }
     sp = TeamSplit();
   }
   out.diag.resize(out.rows.size());

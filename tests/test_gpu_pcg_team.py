@@ -185,3 +185,12 @@ def test_explicit_residency_keeps_the_grid_wide_kernel(resident, b200):
         p.backwardEuler(wl.h, 2, tol=1e-12)
         out.append(p.getStates()[0])
     assert all(np.array_equal(a, b) for a, b in zip(*out))
+
+
+@pytest.mark.parametrize("cells", [(10, 2, 2), (20, 6, 6)])
+def test_teams_hold_no_arrays_of_the_grid_wide_kernel(cells, b200):
+    """Where S fits the CTAs, the teams' tables take less device memory than the vectors and lists they replace."""
+    wl = _beam(L.ELEM_TET, cells, NH)
+    team, grid = (FemPack([wl.model()], precision=L.PREC_FP64, options=o)
+                  for o in ({}, {L.OPT_PCG_SPLIT: L.SPLIT_CONTIGUOUS}))
+    assert team.deviceBytes() < grid.deviceBytes(), (team.deviceBytes(), grid.deviceBytes())
