@@ -62,6 +62,8 @@ cudaError_t dalloc(Engine& eng, T** ptr, size_t count) {
   if (e == cudaSuccess) {
     eng.allocations.push_back((void*)*ptr);
     eng.device_bytes += count * sizeof(T);
+  } else {
+    eng.out_of_memory = e == cudaErrorMemoryAllocation;
   }
   return e;
 }
@@ -93,8 +95,9 @@ void free_pack(Engine& eng) {
   eng.have_matrix = false;
 }
 
-int build_pack(Engine& eng) {
+static int build_pack_with(Engine& eng, bool teams) {
   free_pack(eng);
+  eng.team = eng.out_of_memory = false;
   const int M = (int)eng.models.size();
   if (M == 0) return fail(&eng, B200FEM_ERR_STATE, "no model defined");
   for (auto& m : eng.models) {
@@ -779,7 +782,7 @@ int build_pack(Engine& eng) {
   // not depend on it (40x10x10 hex beam: 2 ms beside 4).
   TeamHost team;
   std::future<bool> planned = std::async([&] {
-    return eng.opt_split == 0 && eng.opt_resident == 0 &&
+    return teams && eng.opt_split == 0 && eng.opt_resident == 0 &&
            plan_team(eng, gmax, prow, eng.factored ? s1_col : col, eng.factored ? s1_diag : blk_diag,
                      eng.factored && !dil_nodes.empty(), team);
   });
@@ -1055,6 +1058,16 @@ int build_pack(Engine& eng) {
   if (eng.team) CK(prepare_team(eng));
   eng.built = true;
   return B200FEM_OK;
+}
+
+int build_pack(Engine& eng) {
+  const int st = build_pack_with(eng, true);
+  if (st == B200FEM_OK || !eng.team || !eng.out_of_memory) return st;
+  // Teams of a large model keep a second copy of the blocks that exceed their
+  // shared memory (60x30x30 hex block, FP64: 576 MB against 475): where that
+  // is too much, the grid-wide kernel.
+  cudaGetLastError();  // (no later launch is to report it)
+  return build_pack_with(eng, false);
 }
 
 }  // namespace b200fem

@@ -446,6 +446,7 @@ struct Engine {
   std::shared_ptr<HostStage> stage;
   std::vector<void*> allocations;
   size_t device_bytes = 0;  // sum of the allocations above
+  bool out_of_memory = false;  // an allocation of the last build failed for want of memory
 };
 
 // setup.cpp

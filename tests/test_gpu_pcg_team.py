@@ -194,3 +194,31 @@ def test_teams_hold_no_arrays_of_the_grid_wide_kernel(cells, b200):
     team, grid = (FemPack([wl.model()], precision=L.PREC_FP64, options=o)
                   for o in ({}, {L.OPT_PCG_SPLIT: L.SPLIT_CONTIGUOUS}))
     assert team.deviceBytes() < grid.deviceBytes(), (team.deviceBytes(), grid.deviceBytes())
+
+
+def test_grid_wide_kernel_where_teams_exceed_the_memory(b200):
+    """A large model's teams hold a copy of the blocks that stream: with device memory for the grid-wide kernel's arrays
+    but not for that copy, the model builds and steps as it does with that kernel."""
+    import torch
+
+    wl = _beam(L.ELEM_HEX, (60, 30, 30), NH)
+    x, v = _state(wl)
+
+    def step(options):
+        p = FemPack([wl.model()], precision=L.PREC_FP64, options=options)
+        p.setStates([x], [v])
+        p.backwardEuler(wl.h, 1, tol=1e-8)
+        out = p.getStates()[0], p.option(L.OPT_PCG_SPLIT), p.deviceBytes()
+        p.close()
+        return out
+
+    _, split, team_bytes = step({})
+    ref, _, grid_bytes = step({L.OPT_PCG_SPLIT: L.SPLIT_CONTIGUOUS})
+    assert split == L.SPLIT_TEAM and team_bytes - grid_bytes > 64 << 20, (team_bytes, grid_bytes)
+    free = torch.cuda.mem_get_info()[0]
+    hold = torch.empty(free - (team_bytes + grid_bytes) // 2, dtype=torch.uint8, device="cuda")
+    got, split, _ = step({})
+    del hold
+    torch.cuda.empty_cache()
+    assert split == L.SPLIT_CONTIGUOUS
+    assert all(np.array_equal(a, b) for a, b in zip(got, ref))
