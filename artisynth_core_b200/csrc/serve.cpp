@@ -144,7 +144,9 @@ struct b200fem_server {
     return B200FEM_OK;
   }
 
-  int build(const std::vector<int>& batch) {
+  // teams false: with the PCG of one split for all models, which needs less
+  // memory where a large model's teams stream
+  int build(const std::vector<int>& batch, bool teams = true) {
     auto slot = std::make_unique<Slot>();
     b200fem_handle h = b200fem_create(&cfg);
     if (!h) return fail(B200FEM_ERR_CUDA, std::string("pack: ") + b200fem_last_error(nullptr));
@@ -168,8 +170,18 @@ struct b200fem_server {
       int rc = b200fem_set_option(h, kv.first, kv.second);
       if (rc != B200FEM_OK) return bail(rc);
     }
-    int rc = b200fem_build(h);
+    int rc = B200FEM_OK;
+    if (!teams) rc = b200fem_set_option(h, B200FEM_OPT_PCG_SPLIT, batch.size() > 1 ? 2 : 1);
+    if (rc == B200FEM_OK) rc = b200fem_build(h);
     if (rc != B200FEM_OK) return bail(rc);
+    unsigned long long nb = 0;
+    b200fem_memory_usage(h, &nb);
+    int split = 0;
+    b200fem_get_option(h, B200FEM_OPT_PCG_SPLIT, &split);
+    if (nb > budget && split == 4) {
+      b200fem_destroy(h);
+      return build(batch, false);
+    }
     size_t total = 0;
     for (size_t i = 0; i < batch.size(); i++) {
       int off = 0, nn = 0, na = 0;
@@ -204,8 +216,6 @@ struct b200fem_server {
       }
       if ((rc = b200fem_set_state(h, x.data(), v.data())) != B200FEM_OK) return bail(rc);
     }
-    unsigned long long nb = 0;
-    b200fem_memory_usage(h, &nb);
     double elems = 0;
     for (int m : batch) elems += pool[m].n_elems;
     calibrate(elems, (double)nb);

@@ -212,6 +212,14 @@ class FemServer:
             else:
                 pack = FemPack(models, precision=self.precision, device=self.device)
                 pack.engine()
+            if pack.deviceBytes() > self.budget:
+                # too large for the budget: once more without the teams' copy
+                # of the blocks that a large model streams
+                pack.close()
+                split = L.SPLIT_STRIDED if len(models) > 1 else L.SPLIT_CONTIGUOUS
+                pack = FemPack(models, precision=self.precision, device=self.device,
+                               options={L.OPT_PCG_SPLIT: split})
+                pack.engine()
             if any(m in self.saved for m in batch):
                 xs, vs = [], []
                 for i, m in enumerate(batch):

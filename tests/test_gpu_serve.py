@@ -187,3 +187,30 @@ def test_native_short_poisson_stream(b200):
     assert out["incomplete"] == 0 and out["requests"] > 0
     assert 0 < out["p50_ms"] <= out["p99_ms"]
     srv.close()
+
+
+@pytest.mark.parametrize("native", [False, True])
+def test_budget_below_the_teams_need(native, b200):
+    """A model whose teams stream needs more memory in teams than without: a budget between the two serves it."""
+    from artisynth_core_b200.femmodel import FemPack, NeoHookeanMaterial
+
+    cells = (60, 24, 24)
+    wl = W.Workload("block", L.ELEM_HEX, cells, tuple(0.01 * c for c in cells), 0.04, 5, NeoHookeanMaterial(5e4, 0.4),
+                    1000.0, "xmin", (0.0, 0.0, -9.81), 0.005, 1).build_mesh()
+    need = []
+    for opts in ({}, {L.OPT_PCG_SPLIT: L.SPLIT_CONTIGUOUS}):
+        p = FemPack([wl.model()], precision=L.PREC_MIXED, options=opts)
+        need.append(p.deviceBytes())
+        p.close()
+    assert need[0] > need[1], need
+    srv = (NativeServer if native else FemServer)([wl], budget=sum(need) / 2, tol=1e-8)
+    r = srv.submit(0, 2)
+    for _ in range(4):
+        srv.tick()
+    if native:
+        assert srv.poll(r)[0] == 2 and srv.stats()["failed"] == 0
+    else:
+        assert not srv.failed and len(srv.done) == 1
+    x = srv.state(0)[0]
+    assert rel_err(x, _alone(wl, 2, L.PREC_MIXED)) <= 1e-6
+    srv.close()
