@@ -222,3 +222,50 @@ def test_grid_wide_kernel_where_teams_exceed_the_memory(b200):
     torch.cuda.empty_cache()
     assert split == L.SPLIT_CONTIGUOUS
     assert all(np.array_equal(a, b) for a, b in zip(got, ref))
+
+
+# what a CTA takes with few CTAs allowed: three component sets (324 and 310 rows in one), steps of S beyond the shared
+# memory, in both precisions and with the factored NODAL matrix
+FULL_CTAS = {
+    "three_sets": (L.ELEM_TET, (9, 5, 5), NH, 1),
+    "three_sets_streamed": (L.ELEM_HEX, (11, 5, 4), NH, 1),
+    "two_ctas_streamed": (L.ELEM_HEX, (16, 5, 5), NH, 2),
+    "quadratic_streamed": (L.ELEM_QUADHEX, (5, 2, 2), NH, 1),
+    "three_sets_nodal": (L.ELEM_TET, (31, 4, 1), MR, 1),
+    "nodal_streamed": (L.ELEM_TET, (12, 5, 5), MR, 2),
+}
+
+
+@pytest.mark.parametrize("precision", [L.PREC_FP64, L.PREC_MIXED])
+@pytest.mark.parametrize("name", list(FULL_CTAS))
+def test_full_ctas_match_grid_wide_kernel(name, precision, b200):
+    elem, cells, mat, ctas = FULL_CTAS[name]
+    wl = _beam(elem, cells, mat)
+    out = []
+    for opts in ({L.OPT_PCG_CTAS: ctas}, {L.OPT_PCG_SPLIT: L.SPLIT_CONTIGUOUS}):
+        p = FemPack([wl.model()], precision=precision, options=opts)
+        p.engine()
+        assert p.option(L.OPT_PCG_SPLIT) == opts.get(L.OPT_PCG_SPLIT, L.SPLIT_TEAM)
+        p.setStates(*([a] for a in _state(wl)))
+        p.backwardEuler(wl.h, 2, tol=1e-12)
+        out.append(p.getStates()[0])
+    (xt, vt), (xg, vg) = out
+    assert rel_err(xt, xg) <= 1e-9 and rel_err(vt, vg) <= 1e-8, (rel_err(xt, xg), rel_err(vt, vg))
+
+
+@pytest.mark.parametrize("precision", [L.PREC_FP64, L.PREC_MIXED])
+def test_pack_of_nodal_and_other_models(precision, b200):
+    """The factored matrix holds for the whole pack: models without NODAL incompressibility run through it beside those
+    with it, queued for few CTAs."""
+    wls = [_beam(e, c, m) for e, c, m in ((L.ELEM_TET, (9, 4, 4), MR), (L.ELEM_TET, (6, 3, 3), NH),
+                                          (L.ELEM_TET, (3, 2, 2), MR), (L.ELEM_TET, (10, 5, 4), NH))]
+    xs, vs = zip(*(_state(w) for w in wls))
+    out = []
+    for opts in ({L.OPT_PCG_CTAS: 3}, {}, {L.OPT_PCG_SPLIT: L.SPLIT_STRIDED}):
+        p = FemPack([w.model() for w in wls], precision=precision, options=opts)
+        p.setStates(xs, vs)
+        p.backwardEuler(wls[0].h, 2, tol=1e-12)
+        out.append(p.getStates())
+    for i in range(len(wls)):
+        for r in out[:2]:
+            assert rel_err(r[i][0], out[2][i][0]) <= 1e-9 and rel_err(r[i][1], out[2][i][1]) <= 1e-8, i

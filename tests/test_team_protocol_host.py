@@ -77,6 +77,14 @@ def emu(tmp_path_factory):
 
 SOLVES = {  # grids, stiffness, dil, fp32, CTAs, shared memory KB, variant, what the plan has to show
     "one_cta": ("4x3x3", "30", 0, 0, 1, 227, 0, {"sets": "1", "team": "1"}),
+    "three_sets": ("9x6x6", "10", 0, 0, 1, 227, 0, {"sets": "3", "team": "1"}),
+    "three_sets_fp32": ("9x6x6", "10", 0, 1, 1, 227, 0, {"sets": "3", "team": "1"}),
+    "three_sets_nodal": ("31x5x2", "10", 1, 0, 1, 227, 0, {"sets": "3", "team": "1"}),
+    "three_sets_nodal_fp32": ("31x5x2", "10", 1, 1, 1, 227, 0, {"sets": "3", "team": "1"}),
+    "streamed_classic": ("9x6x6", "10", 0, 0, 1, 100, 1, {"sets": "3", "kept": "30", "streamed": "200"}),
+    "streamed_pipelined": ("9x6x6", "10", 0, 0, 1, 100, 2, {"sets": "3", "kept": "30", "streamed": "200"}),
+    "team_of_two": ("10x10x9", "10", 0, 1, 2, 227, 0, {"sets": "3", "team": "2"}),
+    "nodal_team_streamed": ("8x8x8", "10", 1, 0, 4, 110, 0, {"sets": "1", "team": "4"}),
 }
 
 
