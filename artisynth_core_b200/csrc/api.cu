@@ -1923,7 +1923,7 @@ int backward_euler_steps(Engine& eng, const b200fem_step_params* p, int nsteps, 
       if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(eng.ev[0], eng.stream, ext);
       if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(eng.ev_pool[0], eng.stream, ext);
       if (ce == cudaSuccess) ce = launch_assemble(eng, false);
-        if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(eng.ev_pool[1], eng.stream, ext);
+      if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(eng.ev_pool[1], eng.stream, ext);
       if (ce == cudaSuccess) ce = launch_solve(eng, max_iter);
       if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(eng.ev_pool[2], eng.stream, ext);
       if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(eng.ev[1], eng.stream, ext);
