@@ -637,6 +637,7 @@ class FemPack:
         return self._engine
 
     def close(self):
+        self.__dict__.pop("_join_buf", None)
         if self._engine is not None:
             self._engine.close()
             self._engine = None
