@@ -9,6 +9,7 @@
 // barrier with a count waits for that many arrivals, whoever has left.
 #pragma once
 
+#include <setjmp.h>
 #include <ucontext.h>
 
 #include <cstdint>
@@ -31,7 +32,8 @@ struct Dim {
 };
 struct Cta;
 struct Fiber {
-  ucontext_t ctx;
+  ucontext_t ctx;  // of its first run; later switches leave the signal mask alone
+  jmp_buf at;
   Cta* cta = nullptr;
   int tid = 0;
   enum { kReady, kBlocked, kDone } state = kReady;
@@ -56,7 +58,7 @@ struct Cta {
 struct Machine {
   std::vector<std::unique_ptr<Cta>> ctas;
   std::deque<Fiber*> ready;
-  ucontext_t main;
+  jmp_buf scheduler;
   Fiber* cur = nullptr;
   std::function<void()> body;
   int grid = 0;
@@ -70,7 +72,9 @@ struct Machine {
 };
 inline Machine* M = nullptr;
 
-inline void to_scheduler() { swapcontext(&M->cur->ctx, &M->main); }
+inline void to_scheduler() {
+  if (_setjmp(M->cur->at) == 0) _longjmp(M->scheduler, 1);
+}
 inline void wake(Fiber& f) {
   if (f.state != Fiber::kBlocked) return;
   f.state = Fiber::kReady;
@@ -215,15 +219,15 @@ inline std::string run(Machine& m, int grid, int threads, size_t dyn_bytes, std:
     m.clock_ns += m.clock_step;
     if (++m.resumes > max_resumes) return "no end";
     if (m.before) m.before(*f);
-    if (!f->started) {
-      f->started = true;
-      getcontext(&f->ctx);
-      f->ctx.uc_stack.ss_sp = f->stack.get();
-      f->ctx.uc_stack.ss_size = kStack;
-      f->ctx.uc_link = &m.main;
-      makecontext(&f->ctx, (void (*)())fiber_main, 0);
-    }
-    swapcontext(&m.main, &f->ctx);
+    if (_setjmp(m.scheduler) != 0) continue;
+    if (f->started) _longjmp(f->at, 1);  // (across stacks: built without the fortified longjmp)
+    f->started = true;
+    getcontext(&f->ctx);
+    f->ctx.uc_stack.ss_sp = f->stack.get();
+    f->ctx.uc_stack.ss_size = kStack;
+    f->ctx.uc_link = nullptr;
+    makecontext(&f->ctx, (void (*)())fiber_main, 0);
+    setcontext(&f->ctx);
   }
   for (auto& c : m.ctas)
     if (c->alive > 0) {

@@ -315,8 +315,9 @@ static int scenario_slow_warp(char** v) {
   return 0;
 }
 
-// Two models, three CTAs, a random interleaving; an error is recorded after
-// `at` scheduling steps (0: never): "random <seed> <at> <variant> <dil>"
+// Three models, three CTAs, a random interleaving; an error is recorded after
+// `at` scheduling steps (0: never).  A second solve follows, after an error
+// with tickets, tags and packets cleared: "random <seed> <at> <variant> <dil>"
 static int scenario_random(char** v) {
   Problem P;
   const unsigned seed = (unsigned)atoi(v[0]);
@@ -332,6 +333,20 @@ static int scenario_random(char** v) {
     if (at > 0 && (long)m.resumes >= at) P.flags[0] = B200FEM_ERR_INVALID_ARG;
   };
   report(P, launch(P, m));
+  if (P.flags[0] != 0) {
+    P.flags[0] = 0;
+    P.ticket = 0;
+    std::fill(P.base.begin(), P.base.end(), 0u);
+    for (auto* v : {&P.row_pk, &P.part_pk, &P.t_pk}) std::fill(v->begin(), v->end(), 0.0);
+  }
+  for (size_t i = 0; i < P.b.size(); i++) {
+    P.b[i] = -2 * P.b[i] + 0.1;
+    P.x[i] = 0.01 * P.b[i];
+  }
+  emu::Machine m2;
+  m2.choose = m.choose;
+  const std::string hang = launch(P, m2);
+  printf("again %s\nagain_flag %d\nagain_residual %.17g\n", hang.empty() ? "yes" : hang.c_str(), P.flags[0], residual(P));
   return 0;
 }
 
