@@ -184,7 +184,7 @@ inline void fiber_main() {
 // Runs `body` on grid x threads; empty when every thread ended, else where
 // they hang.
 inline std::string run(Machine& m, int grid, int threads, size_t dyn_bytes, std::function<void()> body,
-                       uint64_t max_resumes = 100000000ull) {
+                       uint64_t max_resumes = 20000000ull) {
   M = &m;
   m.body = std::move(body);
   m.grid = grid;

@@ -316,7 +316,8 @@ static int scenario_slow_warp(char** v) {
 }
 
 // Three models, three CTAs, a random interleaving; an error is recorded after
-// `at` scheduling steps (0: never).  A second solve follows, after an error
+// `at` scheduling steps (0: never; -1: row 0 has a singular diagonal block, and
+// its warp runs ahead).  A second solve follows, after an error
 // with tickets, tags and packets cleared: "random <seed> <at> <variant> <dil>"
 static int scenario_random(char** v) {
   Problem P;
@@ -325,6 +326,13 @@ static int scenario_random(char** v) {
   make(P, {{9, 6, 5}, {3, 2, 2}, {4, 3, 3}}, {4.0, 1.0, 2.0}, 1e-6, atoi(v[3]) != 0, seed);
   if (!plan(P, 3, false)) return 2;
   P.a.variant = atoi(v[2]);
+  const std::vector<double> S = P.S;
+  size_t bad = 0;  // where row 0 lies among the slots' rows
+  while (P.th.rows[bad] != 0) bad++;
+  if (at < 0) {
+    std::fill_n(&P.S[9 * (size_t)P.diag[0]], 9, 0.0);
+    std::fill(P.kp.begin(), P.kp.begin() + P.eng.row_off[1], 0.0);
+  }
   std::mt19937 rng(seed);
   emu::Machine m;
   // runs of one fiber's neighbours, then a jump: warps drift far apart
@@ -332,7 +340,16 @@ static int scenario_random(char** v) {
   m.before = [&](emu::Fiber&) {
     if (at > 0 && (long)m.resumes >= at) P.flags[0] = B200FEM_ERR_INVALID_ARG;
   };
+  if (at < 0)
+    m.rank = [&](const emu::Fiber& f) {
+      auto& s = f.cta->shared["s_slot"];
+      if (s.empty() || m.resumes > 200000) return 1;  // (others poll for what this CTA publishes)
+      const TeamSlot& sl = *(const TeamSlot*)(((uintptr_t)s.data() + 15) & ~(uintptr_t)15);
+      if ((int)bad < sl.r0 || (int)bad >= sl.r0 + sl.nloc) return 1;
+      return f.warp() == ((int)bad - sl.r0) % kSetRows / 10 ? 1 : 0;
+    };
   report(P, launch(P, m));
+  P.S = S;
   if (P.flags[0] != 0) {
     P.flags[0] = 0;
     P.ticket = 0;

@@ -68,7 +68,7 @@ def emu(tmp_path_factory):
     exe = build(str(tmp_path_factory.mktemp("emu")))
 
     def run(*args):
-        r = subprocess.run([exe, *map(str, args)], capture_output=True, text=True, timeout=600)
+        r = subprocess.run([exe, *map(str, args)], capture_output=True, text=True, timeout=120)
         assert r.returncode == 0, (r.returncode, r.stderr)
         return dict(line.split(" ", 1) for line in r.stdout.splitlines())
 
@@ -127,12 +127,14 @@ def test_lost_packets_of_a_complete_team_time_out(emu):
 
 
 @pytest.mark.parametrize("seed", [0, 1, 2, 5])
-@pytest.mark.parametrize("at", [0, 100000])
+@pytest.mark.parametrize("at", [0, 100000, -1])
 def test_random_interleavings(seed, at, emu):
-    """Three models on three CTAs, with and without an error recorded on the way: every thread ends, and the solve that
+    """Three models on three CTAs, with and without an error recorded or found on the way: every thread ends, and the solve that
     follows is right."""
     out = emu("random", seed, at, seed % 3, seed // 3)
     assert out["ended"] == "yes", out
+    if at < 0:
+        assert out["flag"] == str(L.ERR_INVALID_ARG), out
     if at == 0:
         assert out["flag"] == "0" and float(out["residual"]) <= 1e-6 * (1 + 1e-3), out
     assert out["again"] == "yes" and out["again_flag"] == "0", out
